@@ -147,3 +147,37 @@ def tolerance(case):
     # result to the type already costs 1.6e-3 and 2.0e-4; the rest is the rounding of the probabilities).
     # Four times that:
     return {"rel": 1e-2, "max": 0.2} if case["dtype"] == "bf16" else {"rel": 1.5e-3, "max": 1.5e-2}
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, in 64 bits and without an intermediate rounding."""
+    dev = torch.device("cuda", torch.cuda.current_device())
+    q, k, v, gq, gk, cos, sin = (None if t is None else t.to(dev) for t in prepare(case, seed)["in"])
+    B, S, Hq, Hkv, D = (case[n] for n in ("B", "S", "Hq", "Hkv", "D"))
+    if cos is not None:
+        cos, sin = cos.reshape(S, D).double(), sin.reshape(S, D).double()
+
+    def rows(x, gamma):
+        x = x.double()
+        y = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * gamma.double()
+        if cos is None:
+            return y
+        lo, hi = y[..., : D // 2], y[..., D // 2:]
+        return y * cos + torch.cat((-hi, lo), -1) * sin
+
+    out = torch.empty(B, Hq, S, D, dtype=torch.float64, device=dev)
+    step = max(1, min(S, (1 << 28) // S))  # query rows at a time: 2 GB of scores
+    for b in range(B):
+        for h in range(Hq):
+            g = h // (Hq // Hkv)
+            if h % (Hq // Hkv) == 0:
+                kt, vv = rows(k[b, g], gk).t(), v[b, g].double()
+            qn = rows(q[b, h], gq) * D ** -0.5
+            for r in range(0, S, step):
+                n = min(step, S - r)
+                keys = r + n if case["causal"] else S  # later keys are masked for all of these rows
+                s = qn[r: r + n] @ kt[:, :keys]
+                if case["causal"]:
+                    s.masked_fill_(torch.ones(n, keys, dtype=torch.bool, device=dev).triu_(r + 1), -math.inf)
+                out[b, h, r: r + n] = torch.softmax(s, -1) @ vv
+    return out.transpose(1, 2).reshape(B, S, Hq * D) if case["entry"] == "layer" else out
