@@ -181,16 +181,13 @@ attn_fwd_persist256_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
         const int r = tid;
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
         const float cs = a.scale_log2e;
-        const float inv_c = 1.f / cs;
         int g = 0;  // sub-blocks processed so far (all tiles)
         for (int n = 0; !fail; ++n) {
             const int idx = p2_take_item<true>(c, n, lane, fail);
             if (idx < 0) break;
             const P2Item it = p2_decode(idx, a);
             const int row = it.m0 + r;
-            float m_used = -INFINITY, den = 0.f;
-            PolyBase pb;
-            pb.set(0.f, inv_c);
+            RowSoftmax rs;
             for (int jj = 0; jj < it.nsub; ++jj) {
                 const int gg = g + jj;
                 const int buf = gg & 1;
@@ -200,78 +197,12 @@ attn_fwd_persist256_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 if (tid == 0 && jj == max(0, it.nsub - kP2ClaimAhead)) mbar_arrive(&c->near_end);
                 if (!mbar_wait_abortable(c->s_full + buf, (gg >> 1) & 1, s_abort)) { fail = kStatusP2SFull; break; }
                 tc_fence_after();
-                uint32_t sr[2][32];
-                tmem_ld32(lane_base + col_sb, sr[0]);
-                tmem_ld32(lane_base + col_sb + 32, sr[1]);
-                tmem_wait_ld();
-                const bool need_mask = (n0 + kSub > a.S) || (a.causal && (n0 + kSub - 1 > it.m0));
-                if (need_mask) {
-#pragma unroll
-                    for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int col = n0 + q2 * 32 + i;
-                            if (col >= a.S || (a.causal && col > row)) sr[q2][i] = 0xff800000u;  // -inf
-                        }
-                }
-                float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-                for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        mx0 = max3(mx0, __uint_as_float(sr[q2][i]), __uint_as_float(sr[q2][i + 1]));
-                        mx1 = max3(mx1, __uint_as_float(sr[q2][i + 2]), __uint_as_float(sr[q2][i + 3]));
-                    }
-                const float m_blk = fmaxf(mx0, mx1) * cs;
-                // move the exponent base only when the maximum grew by more than the threshold
-                const bool grow = m_blk > m_used + kRescaleThreshold;
-                float alpha = 1.f;
-                if (grow) {
-                    alpha = fast_exp2(m_used - m_blk);  // 0 on the first sub-block
-                    m_used = m_blk;
-                    den *= alpha;
-                    pb.set(m_used, inv_c);
-                }
-                const float neg_m = -m_used;
-                const f32x2 c2 = f2_pack(cs, cs), nm2 = f2_pack(neg_m, neg_m);
-                f32x2 psum = f2_pack(0.f, 0.f);
-#pragma unroll
-                for (int q2 = 0; q2 < 2; ++q2) {
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float s0 = __uint_as_float(sr[q2][2 * i]), s1 = __uint_as_float(sr[q2][2 * i + 1]);
-                        float p0, p1;
-                        if ((kPolyPairMask >> (q2 * 16 + i)) & 1u) {
-                            exp2_poly2_scaled(s0, s1, c2, pb, p0, p1);
-                        } else {
-                            float x0, x1;
-                            f2_unpack(f2_fma(f2_pack(s0, s1), c2, nm2), x0, x1);
-                            p0 = fast_exp2(x0);
-                            p1 = fast_exp2(x1);
-                        }
-                        psum = f2_add(psum, f2_pack(p0, p1));
-                        pk[i] = Num<T>::pack(p0, p1);
-                    }
-                    tmem_st16(lane_base + col_sb + q2 * 16, pk);  // P overwrites its S (already in registers)
-                }
-                float ps0, ps1;
-                f2_unpack(psum, ps0, ps1);
-                den += ps0 + ps1;
-                if (jj > 0 && __any_sync(0xffffffffu, grow)) {
-                    // O may only be touched once the previous P V has completed (pv_done alternates between two
-                    // barriers, so a phase cannot be lapped: P V of g+1 needs this P)
-                    if (!mbar_wait_abortable(c->pv_done + ((gg - 1) & 1), ((gg - 1) >> 1) & 1, s_abort)) { fail = kStatusP2PvDone; break; }
-                    tc_fence_after();
-#pragma unroll
-                    for (int q4 = 0; q4 < D / 32; ++q4) {
-                        uint32_t o[32];
-                        tmem_ld32(lane_base + kColO + q4 * 32, o);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st32(lane_base + kColO + q4 * 32, o);
-                    }
+                const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= it.m0);
+                if (!plain || !softmax_ordinary<T, false>(lane_base + col_sb, cs, rs)) {
+                    const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
+                    rs = softmax_general<D, T>(lane_base + col_sb, lane_base + kColO, cs, lim, rs, jj > 0 ? c->pv_done + ((gg - 1) & 1) : nullptr,
+                                               ((gg - 1) >> 1) & 1, s_abort);
+                    if (!rs.ok) { fail = kStatusP2PvDone; break; }
                 }
                 tmem_wait_st();
                 tc_fence_before();
@@ -284,7 +215,7 @@ attn_fwd_persist256_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
             // (it signals o_free after reading them); a tile of one or two sub-blocks can get here before any of
             // its P V has been issued, so this wait is not implied by the pipeline.
             if (n > 0 && !mbar_wait_abortable(&c->o_free, (n - 1) & 1, s_abort)) { fail = kStatusP2OFree; break; }
-            c->den[r] = den;
+            c->den[r] = rs.den;
             __syncwarp();
             if (lane == 0) mbar_arrive(&c->den_full);
         }

@@ -46,7 +46,6 @@ constexpr int kWsStages = 2;
 constexpr int kWsTileBytes = 2 * kBoxBytes;  // 128 rows x 128 columns of 16-bit values
 constexpr int kWsSmemBytes = (2 + 2 * kWsStages) * kWsTileBytes + 1024 + 512;  // tiles, alignment slack, barriers
 constexpr int kWsSmemBytesFactored = kWsSmemBytes + 1024;  // + inverse RMS of the Q rows (factored form only)
-constexpr float kRescaleThreshold = 8.0f;  // log2 units
 constexpr int kSub = 64;                    // keys per sub-block
 
 __device__ __forceinline__ bool mbar_wait_abortable(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -113,7 +112,7 @@ __device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
     return d;
 }
 
-// 2^x for x <= 0 on the FMA pipe (relieves the MUFU unit, which would otherwise
+// 2^x for x <= kGrowLimit on the FMA pipe (relieves the MUFU unit, which would otherwise
 // limit the kernel): n = round(x), f = x - n in [-0.5, 0.5], 2^f by a cubic
 // (max relative error 7.5e-5, far below the 16-bit rounding of P), 2^n by an
 // integer add into the exponent field.  x is clamped at -125 so the exponent
@@ -135,50 +134,123 @@ __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float&
     p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(r1) << 23));
 }
 
-// The polynomial with the score scaling folded in.  The softmax's exponent base m is an
-// arbitrary float; the polynomial works from the nearest integer mi = rint(m) (so that
-// magic - mi is exact) and its coefficients carry the factor 2^(mi - m), which makes both
-// exp paths produce 2^(s*c - m):
-//   fr = s*c + (magic - mi)     -> n + magic, n = round(s*c - mi)     (one packed FMA)
-//   u  = (magic - mi) - fr      -> -(n + mi), exact
-//   f  = s*c + u                -> (s*c - mi) - n in [-0.5, 0.5]      (one packed FMA)
-//   p  = 2^(mi - m) * cubic(f) * 2^n
-// s is clamped from below at s_min = (mi - 125)/c, which keeps n >= -125 (no exponent
-// underflow) and turns a masked -inf score into ~2^-125.
-struct PolyBase {
-    f32x2 magic_minus_mi, k0, k1, k2, k3;
-    float s_min;
-    __device__ __forceinline__ void set(float m, float inv_c) {
-        const float mi = rintf(m);
-        const float k = fast_exp2(mi - m);
-        magic_minus_mi = f2_pack(12582912.f - mi, 12582912.f - mi);
-        k0 = f2_pack(0.9999280572f * k, 0.9999280572f * k);
-        k1 = f2_pack(0.6932609677f * k, 0.6932609677f * k);
-        k2 = f2_pack(0.2426111251f * k, 0.2426111251f * k);
-        k3 = f2_pack(0.0551716685f * k, 0.0551716685f * k);
-        s_min = (mi - 125.f) * inv_c;
-    }
-};
-__device__ __forceinline__ void exp2_poly2_scaled(float s0, float s1, f32x2 c2, const PolyBase& pb, float& p0,
-                                                  float& p1) {
-    const f32x2 sv = f2_pack(fmaxf(s0, pb.s_min), fmaxf(s1, pb.s_min));
-    const f32x2 fr = f2_fma(sv, c2, pb.magic_minus_mi);
-    const f32x2 f = f2_fma(sv, c2, f2_sub(pb.magic_minus_mi, fr));
-    f32x2 p = f2_fma(f, pb.k3, pb.k2);
-    p = f2_fma(f, p, pb.k1);
-    p = f2_fma(f, p, pb.k0);
-    float r0, r1, q0, q1;
-    f2_unpack(fr, r0, r1);
-    f2_unpack(p, q0, q1);
-    p0 = __int_as_float(__float_as_int(q0) + (__float_as_int(r0) << 23));
-    p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(r1) << 23));
-}
-
 // Which pairs of a 32-pair sub-block row go through the polynomial (the rest use MUFU ex2).
 #ifndef KF_POLY_MASK
 #define KF_POLY_MASK 0x88888888u  // every 4th pair: 25 %
 #endif
 constexpr uint32_t kPolyPairMask = KF_POLY_MASK;
+
+// ---- softmax of one 64-key sub-block of one row
+// A row's exponent base is the maximum of its first sub-block and from then on of each one with a score more than
+// kGrowLimit above the base, which keeps every probability at or below 2^8.  (Not rounded to a whole number: the
+// row's largest probability is then exactly 1, and in short rows its rounding is most of the error.)
+constexpr float kGrowLimit = 8.0f;  // log2 units
+struct RowSoftmax {
+    float m = -INFINITY;  // exponent base (log2 units)
+    float den = 0.f;      // sum of the probabilities so far, relative to the base
+    bool ok = true;       // false: a bounded wait ran out
+};
+
+// Probabilities of the row's 64 scores against base m, packed into pk; returns their sum.
+template <typename T>
+__device__ __forceinline__ float exp_sub_block(const uint32_t (&sr)[2][32], float c, float m, uint32_t (&pk)[32]) {
+    const f32x2 c2 = f2_pack(c, c), nm2 = f2_pack(-m, -m);
+    f32x2 psum = f2_pack(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        const float u0 = __uint_as_float(sr[i / 16][2 * (i % 16)]), u1 = __uint_as_float(sr[i / 16][2 * (i % 16) + 1]);
+        float x0, x1, p0, p1;
+        f2_unpack(f2_fma(f2_pack(u0, u1), c2, nm2), x0, x1);
+        if ((kPolyPairMask >> i) & 1u) {
+            exp2_poly2(x0, x1, p0, p1);
+        } else {
+            p0 = fast_exp2(x0);
+            p1 = fast_exp2(x1);
+        }
+        psum = f2_add(psum, f2_pack(p0, p1));
+        pk[i] = Num<T>::pack(p0, p1);
+    }
+    float a0, a1;
+    f2_unpack(psum, a0, a1);
+    return a0 + a1;
+}
+
+// Multiply the row's D output columns in TMEM by alpha.
+template <int D> __device__ __forceinline__ void rescale_output(uint32_t taddr, float alpha) {
+#pragma unroll
+    for (int q4 = 0; q4 < D / 32; ++q4) {
+        uint32_t o[32];
+        tmem_ld32(taddr + q4 * 32, o);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+        tmem_st32(taddr + q4 * 32, o);
+    }
+}
+
+// The general sub-block: the row's first (`prev_pv` null: the base is set from its maximum), one of which only the
+// first `lim` scores count, or one whose scores have left the base behind.  Takes the maximum, moves the base if it has
+// to, computes and stores P; when a row of the warp moved its base after the first sub-block, waits for the previous
+// P V and multiplies the output so far by alpha.  `ok` is false if that wait failed.
+// Not inlined: these are few of a long row's sub-blocks, and the loop of the others has to stay one short straight run of
+// code.  B200, against the same kernels with mask, maximum and rescale inside the loop (2 s of back-to-back calls):
+// B=16 S=4096 32/8 heads 2358 -> 2320 us, B=1 S=16384 2049 -> 2015 us, B=4 S=2048 193.4 -> 190.8 us.
+template <int D, typename T>
+__device__ __noinline__ RowSoftmax softmax_general(uint32_t taddr, uint32_t taddr_o, float c, int lim, RowSoftmax rs,
+                                                   uint64_t* prev_pv, uint32_t parity, volatile int* abort_flag) {
+    uint32_t sr[2][32], pk[32];
+    tmem_ld32(taddr, sr[0]);
+    tmem_ld32(taddr + 32, sr[1]);
+    tmem_wait_ld();
+    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int i = 0; i < 64; i += 2) {
+        if (i >= lim) sr[i / 32][i % 32] = 0xff800000u;  // -inf
+        if (i + 1 >= lim) sr[i / 32][i % 32 + 1] = 0xff800000u;
+        mx[(i / 2) & 1] = max3(mx[(i / 2) & 1], __uint_as_float(sr[i / 32][i % 32]), __uint_as_float(sr[i / 32][i % 32 + 1]));
+    }
+    const float m_blk = fmaxf(mx[0], mx[1]) * c;
+    const bool grow = m_blk > rs.m + kGrowLimit;
+    float alpha = 1.f;
+    if (grow) {
+        alpha = fast_exp2(rs.m - m_blk);  // 0 on the first sub-block
+        rs.m = m_blk;
+    }
+    const float sum = exp_sub_block<T>(sr, c, rs.m, pk);
+    tmem_st32(taddr, pk);  // P overwrites its S
+    rs.den = rs.den * alpha + sum;
+    if (prev_pv != nullptr && __any_sync(0xffffffffu, grow)) {
+        // O may only be touched once the previous P V has completed.  (pv_done alternates between two barriers, so a
+        // phase cannot be lapped: the next P V needs this sub-block's P.)
+        rs.ok = __all_sync(0xffffffffu, mbar_wait_abortable(prev_pv, parity, abort_flag)) != 0;
+        tc_fence_after();
+        if (rs.ok) rescale_output<D>(taddr_o, alpha);
+    }
+    return rs;
+}
+
+// An ordinary sub-block (all 64 scores count, the base is set): P is computed against the base as it stands; false, with
+// nothing stored, when a score of the warp lies too far above it.  The exponentials do not depend on the maximum, so
+// the two chains overlap.  MAX_FIRST orders the source for the compiler: with two softmax warps per scheduler (D = 128)
+// the maximum first is 2-5 % of a launch faster, with one (D = 256) the exponentials first by 3 %.
+template <typename T, bool MAX_FIRST>
+__device__ __forceinline__ bool softmax_ordinary(uint32_t taddr, float c, RowSoftmax& rs) {
+    uint32_t sr[2][32], pk[32];
+    tmem_ld32(taddr, sr[0]);
+    tmem_ld32(taddr + 32, sr[1]);
+    tmem_wait_ld();
+    float sum = 0.f;
+    if (!MAX_FIRST) sum = exp_sub_block<T>(sr, c, rs.m, pk);
+    float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int i = 0; i < 64; i += 2)
+        mx[(i / 2) & 3] = max3(mx[(i / 2) & 3], __uint_as_float(sr[i / 32][i % 32]), __uint_as_float(sr[i / 32][i % 32 + 1]));
+    if (__any_sync(0xffffffffu, fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * c > rs.m + kGrowLimit)) return false;
+    if (MAX_FIRST) sum = exp_sub_block<T>(sr, c, rs.m, pk);
+    tmem_st32(taddr, pk);  // P overwrites its S
+    rs.den += sum;
+    return true;
+}
 
 struct WsTile {
     int h, m0, nsub;
@@ -319,7 +391,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 __syncwarp();
                 if (lane == 0) mbar_arrive(q_ready + t);
             }
-            float m_used = -INFINITY, den = 0.f;
+            RowSoftmax rs;
             float c_row = a.scale_log2e;
             if constexpr (FACTORED) {
                 // every thread of the group takes part, whatever its wait returned, and all follow the vote
@@ -336,81 +408,17 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 if (!s_known_ready &&
                     !mbar_wait_abortable(s_full + 2 * t + buf, (jj >> 1) & 1, s_abort)) { fail = kStatusWsSFull; break; }
                 tc_fence_after();
-                uint32_t sr[2][32];
-                tmem_ld32(lane_base + col_sb, sr[0]);
-                tmem_ld32(lane_base + col_sb + 32, sr[1]);
-                tmem_wait_ld();
-                const bool need_mask = (n0 + kSub > a.S) || (a.causal && (n0 + kSub - 1 > tl.m0));
-                if (need_mask) {
-#pragma unroll
-                    for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int n = n0 + q2 * 32 + i;
-                            if (n >= a.S || (a.causal && n > row)) sr[q2][i] = 0xff800000u;  // -inf
-                        }
-                }
-                float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-                for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        mx0 = max3(mx0, __uint_as_float(sr[q2][i]), __uint_as_float(sr[q2][i + 1]));
-                        mx1 = max3(mx1, __uint_as_float(sr[q2][i + 2]), __uint_as_float(sr[q2][i + 3]));
-                    }
-                const float m_blk = fmaxf(mx0, mx1) * c;
-                // move the exponent base only when the maximum grew by more than the threshold
-                const bool grow = m_blk > m_used + kRescaleThreshold;
-                float alpha = 1.f;
-                if (grow) {
-                    alpha = fast_exp2(m_used - m_blk);  // 0 on the first sub-block
-                    m_used = m_blk;
-                    den *= alpha;
-                }
-                const float neg_m = -m_used;
-                const f32x2 c2 = f2_pack(c, c), nm2 = f2_pack(neg_m, neg_m);
-                f32x2 psum = f2_pack(0.f, 0.f);
-#pragma unroll
-                for (int q2 = 0; q2 < 2; ++q2) {
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        float x0, x1, p0, p1;
-                        f2_unpack(f2_fma(f2_pack(__uint_as_float(sr[q2][2 * i]), __uint_as_float(sr[q2][2 * i + 1])), c2, nm2),
-                                  x0, x1);
-                        if ((kPolyPairMask >> (q2 * 16 + i)) & 1u) {
-                            exp2_poly2(x0, x1, p0, p1);
-                        } else {
-                            p0 = fast_exp2(x0);
-                            p1 = fast_exp2(x1);
-                        }
-                        psum = f2_add(psum, f2_pack(p0, p1));
-                        pk[i] = Num<T>::pack(p0, p1);
-                    }
-                    tmem_st16(lane_base + col_sb + q2 * 16, pk);  // P overwrites its S (already in registers)
+                const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= tl.m0);
+                if (!plain || !softmax_ordinary<T, true>(lane_base + col_sb, c, rs)) {
+                    const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
+                    rs = softmax_general<D, T>(lane_base + col_sb, lane_base + col_o, c, lim, rs, jj > 0 ? pv_done + 2 * t + ((jj - 1) & 1) : nullptr,
+                                               ((jj - 1) >> 1) & 1, s_abort);
+                    if (!rs.ok) { fail = kStatusWsPvDone; break; }
                 }
                 // Probe the next score buffer now: the probe is a shared-memory round trip whose latency
                 // overlaps the store completion and barrier traffic below.
                 s_known_ready = (jj + 1 < tl.nsub) &&
                                 mbar_test_wait(s_full + 2 * t + (buf ^ 1), ((jj + 1) >> 1) & 1);
-                float ps0, ps1;
-                f2_unpack(psum, ps0, ps1);
-                den += ps0 + ps1;
-                if (jj > 0 && __any_sync(0xffffffffu, grow)) {
-                    // O may only be touched once the previous P V has completed.  (pv_done alternates
-                    // between two barriers, so a phase cannot be lapped: P V of jj+1 needs this P.)
-                    if (!mbar_wait_abortable(pv_done + 2 * t + ((jj - 1) & 1), ((jj - 1) >> 1) & 1, s_abort)) { fail = kStatusWsPvDone; break; }
-                    tc_fence_after();
-#pragma unroll
-                    for (int q4 = 0; q4 < D / 32; ++q4) {
-                        uint32_t o[32];
-                        tmem_ld32(lane_base + col_o + q4 * 32, o);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tmem_st32(lane_base + col_o + q4 * 32, o);
-                    }
-                }
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
@@ -420,7 +428,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             if (!fail && !mbar_wait_abortable(pv_done + 2 * t + ((tl.nsub - 1) & 1), ((tl.nsub - 1) >> 1) & 1, s_abort)) fail = kStatusWsODone;
             if (!fail) {
                 tc_fence_after();
-                const float inv_den = 1.f / den;
+                const float inv_den = 1.f / rs.den;
                 uint8_t* orow = my_q + r * 128;
                 const int sw = r & 7;
 #pragma unroll

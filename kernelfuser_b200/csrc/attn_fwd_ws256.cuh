@@ -198,10 +198,7 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(q_ready);
         }
-        float m_used = -INFINITY, den = 0.f;
-        const float inv_c = 1.f / c;
-        PolyBase pb;
-        pb.set(0.f, inv_c);
+        RowSoftmax rs;
         KF_W1_STAMP(3);
         for (int jj = 0; jj < n_sub && !fail; ++jj) {
             const int buf = jj & 1;
@@ -210,78 +207,12 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             if (!mbar_wait_abortable(s_full + buf, (jj >> 1) & 1, s_abort)) { fail = kStatusWsSFull; break; }
             tc_fence_after();
             if (jj == 0) KF_W1_STAMP(4);
-            uint32_t sr[2][32];
-            tmem_ld32(lane_base + col_sb, sr[0]);
-            tmem_ld32(lane_base + col_sb + 32, sr[1]);
-            tmem_wait_ld();
-            const bool need_mask = (n0 + kSub > a.S) || (a.causal && (n0 + kSub - 1 > m0));
-            if (need_mask) {
-#pragma unroll
-                for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int n = n0 + q2 * 32 + i;
-                        if (n >= a.S || (a.causal && n > row)) sr[q2][i] = 0xff800000u;  // -inf
-                    }
-            }
-            float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2)
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    mx0 = max3(mx0, __uint_as_float(sr[q2][i]), __uint_as_float(sr[q2][i + 1]));
-                    mx1 = max3(mx1, __uint_as_float(sr[q2][i + 2]), __uint_as_float(sr[q2][i + 3]));
-                }
-            const float m_blk = fmaxf(mx0, mx1) * c;
-            // move the exponent base only when the maximum grew by more than the threshold
-            const bool grow = m_blk > m_used + kRescaleThreshold;
-            float alpha = 1.f;
-            if (grow) {
-                alpha = fast_exp2(m_used - m_blk);  // 0 on the first sub-block
-                m_used = m_blk;
-                den *= alpha;
-                pb.set(m_used, inv_c);
-            }
-            const float neg_m = -m_used;
-            const f32x2 c2 = f2_pack(c, c), nm2 = f2_pack(neg_m, neg_m);
-            f32x2 psum = f2_pack(0.f, 0.f);
-#pragma unroll
-            for (int q2 = 0; q2 < 2; ++q2) {
-                uint32_t pk[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float s0 = __uint_as_float(sr[q2][2 * i]), s1 = __uint_as_float(sr[q2][2 * i + 1]);
-                    float p0, p1;
-                    if ((kPolyPairMask >> (q2 * 16 + i)) & 1u) {
-                        exp2_poly2_scaled(s0, s1, c2, pb, p0, p1);
-                    } else {
-                        float x0, x1;
-                        f2_unpack(f2_fma(f2_pack(s0, s1), c2, nm2), x0, x1);
-                        p0 = fast_exp2(x0);
-                        p1 = fast_exp2(x1);
-                    }
-                    psum = f2_add(psum, f2_pack(p0, p1));
-                    pk[i] = Num<T>::pack(p0, p1);
-                }
-                tmem_st16(lane_base + col_sb + q2 * 16, pk);  // P overwrites its S (already in registers)
-            }
-            float ps0, ps1;
-            f2_unpack(psum, ps0, ps1);
-            den += ps0 + ps1;
-            if (jj > 0 && __any_sync(0xffffffffu, grow)) {
-                // O may only be touched once the previous P V has completed.  (pv_done alternates between
-                // two barriers, so a phase cannot be lapped: P V of jj+1 needs this sub-block's P.)
-                if (!mbar_wait_abortable(pv_done + ((jj - 1) & 1), ((jj - 1) >> 1) & 1, s_abort)) { fail = kStatusWsPvDone; break; }
-                tc_fence_after();
-#pragma unroll
-                for (int q4 = 0; q4 < D / 32; ++q4) {
-                    uint32_t o[32];
-                    tmem_ld32(lane_base + kColO + q4 * 32, o);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                    tmem_st32(lane_base + kColO + q4 * 32, o);
-                }
+            const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= m0);
+            if (!plain || !softmax_ordinary<T, D == 128>(lane_base + col_sb, c, rs)) {
+                const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
+                rs = softmax_general<D, T>(lane_base + col_sb, lane_base + kColO, c, lim, rs, jj > 0 ? pv_done + ((jj - 1) & 1) : nullptr,
+                                           ((jj - 1) >> 1) & 1, s_abort);
+                if (!rs.ok) { fail = kStatusWsPvDone; break; }
             }
             tmem_wait_st();
             tc_fence_before();
@@ -294,7 +225,7 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             !mbar_wait_abortable(pv_done + ((n_sub - 1) & 1), ((n_sub - 1) >> 1) & 1, s_abort)) fail = kStatusWsODone;
         if (!fail) {
             tc_fence_after();
-            const float inv_den = 1.f / den;
+            const float inv_den = 1.f / rs.den;
             uint8_t* orow = smem_q + r * 128;
             const int sw = r & 7;
 #pragma unroll
