@@ -15,6 +15,7 @@
 #include "attn_fwd_ws.cuh"
 #include "attn_fwd_persist.cuh"
 #include "attn_fwd_persist256.cuh"
+#include "attn_fwd_pair256.cuh"
 #include "attn_fwd_ws256.cuh"
 #include "prepare_rows.cuh"
 
@@ -328,6 +329,25 @@ int launch_attn_persist256(const CUtensorMap& mq, const CUtensorMap& mk, const C
     return KF_OK;
 }
 
+template <typename T>
+int launch_attn_pair256(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kf::AttnArgs& a0,
+                        cudaStream_t st, bool dependent = false) {
+    auto kern = kf::attn_fwd_pair256_kernel<T>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kf::kPrSmemBytes);
+    if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
+    kf::AttnArgs a = a0;
+    if (int r = sched_slot(&a.sched)) return r;
+    const long long n_mblk = (a.S + kf::kBM - 1) / kf::kBM;
+    const long long items = n_mblk * a.B * (a.Hq / 2);
+    if (items > 0x7fffffffLL) return fail(KF_EINVAL, "too many tiles");
+    const int pairs = sm_count() / 2;
+    const int grid = 2 * (int)(items < pairs ? items : pairs);
+    e = launch_kernel_ex(kern, dim3((unsigned)grid), dim3(kf::kP2Threads), (size_t)kf::kPrSmemBytes, st, dependent, mq, mk, mv, a,
+                         (int)items);
+    if (e != cudaSuccess) return fail(KF_ECUDA, "attention launch failed: %s", cudaGetErrorString(e));
+    return KF_OK;
+}
+
 }  // namespace
 
 
@@ -491,11 +511,21 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
     if (D == 256 && variant == 0 && !factored) {
         // The persistent kernel hides a tile's fixed costs (raw Q copy, transform, copy into TMEM, output store)
         // behind the previous / next tile's main loop; it pays once every SM has a few hundred 64-key sub-blocks
-        // to work through (measured: -11 % time on C5, -2 ... -6 % on its 8/4-GPU shards, +4 ... +18 % on launches
-        // with about a hundred sub-blocks per SM, where the one-launch-per-tile kernel balances better).
+        // to work through (B200, one launch item per tile -> SM pairs: B=8 S=8192 16/8 heads 4222 -> 3502 us, B=1 S=16384
+        // 4/2 heads 473 -> 437; with about a hundred sub-blocks per SM the one-tile kernel balances better: B=1 S=4096
+        // 155 -> 165, B=4 S=1024 82 -> 102).
         const long long n_mblk = (S + kf::kBM - 1) / kf::kBM, n_sub_all = (S + kf::kSub - 1) / kf::kSub;
         const long long per_head = causal ? n_mblk * (n_mblk + 1) : n_mblk * n_sub_all;
         if ((long long)B * Hq * per_head >= kPersist256MinSubBlocksPerSm * sm_count()) variant = 3;
+    }
+    if (D == 256 && variant == 3 && !factored && (Hq / Hkv) % 2 == 0) {
+        // Query heads that share a KV head in even numbers run on SM pairs, 7-13 % faster than one CTA per tile
+        // wherever the persistent form is chosen at all.
+        CUtensorMap mk32, mv64;  // each CTA of a pair loads 32 keys of K and half of the columns of V
+        if (int r = make_map(&mk32, kn, dtype, B, Hkv, S, D, k_sb, k_sh, k_ss, 32)) return r;
+        if (int r = make_map(&mv64, v, dtype, B, Hkv, S, D, v_sb, v_sh, v_ss, 64)) return r;
+        return dtype == KF_BF16 ? launch_attn_pair256<__nv_bfloat16>(mq, mk32, mv64, a, st, dependent && KF_DEPENDENT_PERSIST)
+                                : launch_attn_pair256<__half>(mq, mk32, mv64, a, st, dependent && KF_DEPENDENT_PERSIST);
     }
     if (D == 256 && variant == 3) {
         if (factored) return fail(KF_EINVAL, "the factored form runs on kernels 0, 2 and 5 only");

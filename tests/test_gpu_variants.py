@@ -88,3 +88,20 @@ def test_persistent_kernels_reuse_their_counter_slots():
     kf.check_status()
     for out, ref in outs:
         assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("b,s,hq,hkv,causal,dtype", [
+    (1, 1, 2, 1, True, torch.bfloat16),     # one row, one pair of CTAs
+    (3, 65, 4, 2, False, torch.float16),    # the second sub-block has one key: CTA 1's half of it lies past the end
+    (2, 97, 4, 1, True, torch.bfloat16),    # ... and starts there
+    (16, 300, 16, 4, True, torch.bfloat16), # several items per pair of CTAs, ragged tail
+    (20, 129, 8, 4, False, torch.float16),  # items of three sub-blocks: shorter than the claim distance
+])
+def test_d256_sm_pairs_match_oracle(b, s, hq, hkv, causal, dtype):
+    xs = kf.make_inputs(b, s, hq, hkv, 256, dtype=dtype, theta=1e4, seed=67)
+    ref = orc.oracle_fp32(*xs, causal)
+    out = kf.optimized_attention(*[x.cuda() for x in xs], causal=causal, variant=3)
+    torch.cuda.synchronize()
+    kf.check_status()
+    m = orc.metric(out.cpu(), ref)
+    assert orc.within_tolerance(m), (b, s, hq, hkv, m)
