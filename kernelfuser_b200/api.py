@@ -16,6 +16,7 @@ reached through ctypes; there is no fallback path.
 from __future__ import annotations
 
 import os
+from contextlib import nullcontext
 
 import torch
 
@@ -69,7 +70,28 @@ def selftest_wait_timeout(limit_clocks: int = 100_000, device=None) -> None:
 
 
 def _strides3(t: torch.Tensor):
-    return t.stride(0), t.stride(1), t.stride(2)
+    return t.stride()[:3]
+
+
+# Raw handle of the current stream of a device index: what torch.cuda.current_stream(i).cuda_stream returns, without
+# the Stream object built around it (0.1 against 3.3 us).
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_capability_major = {}  # device index -> compute capability, major
+
+
+def _major(index: int) -> int:
+    m = _capability_major.get(index)
+    if m is None:
+        m = _capability_major[index] = torch.cuda.get_device_capability(index)[0]
+    return m
+
+
+_HERE = nullcontext()
+
+
+def _on_device(index: int):
+    """Context in which device ``index`` is current: nothing to do in the usual case that it is already."""
+    return _HERE if torch._C._cuda_getDevice() == index else torch.cuda.device(index)
 
 
 def _ptr(t):
@@ -138,25 +160,40 @@ def _validate(q, k, v, gq, gk, cos, sin, mode, bn, norm_style, require_contiguou
     if (cos is None) != (sin is None):
         raise ValueError("Provide both rotary tables or neither")
     rotary = cos is not None
-    tensors = (q, k, v, gq, gk) + ((cos, sin) if rotary else ())
-    if any(t.requires_grad for t in tensors):
-        raise ValueError("This API is forward-only")
+    tensors = (q, k, v, gq, gk, cos, sin) if rotary else (q, k, v, gq, gk)
+    for t in tensors:
+        if t.requires_grad:
+            raise ValueError("This API is forward-only")
     if q.ndim != 4 or k.ndim != 4 or k.shape != v.shape:
         raise ValueError("Expected Q [B,Hq,S,D] and K/V [B,Hkv,S,D]")
     b, h, s, d = q.shape
-    if (d not in (128, 256) or min(b, h, s) < 1 or k.shape[0] != b or
-            tuple(k.shape[2:]) != (s, d) or k.shape[1] < 1 or h % k.shape[1]):
+    kb, kh, ks, kd = k.shape
+    if d not in (128, 256) or b < 1 or h < 1 or s < 1 or kb != b or ks != s or kd != d or kh < 1 or h % kh:
         raise ValueError("Expected D=128/256, matching batch/sequence and valid GQA")
-    if tuple(gq.shape) != (d,) or tuple(gk.shape) != (d,) or (
-            rotary and (tuple(cos.shape) != (s, d) or tuple(sin.shape) != (s, d))):
+    if gq.shape != (d,) or gk.shape != (d,) or (rotary and (cos.shape != (s, d) or sin.shape != (s, d))):
         raise ValueError("Expected gamma [D] and optional rotary tables [S,D]")
-    if (q.dtype not in _DTYPES or
-            any(not t.is_cuda or t.device != q.device or t.dtype != q.dtype for t in tensors) or
-            (require_contiguous and any(not t.is_contiguous() for t in tensors))):
+    dtype, index = q.dtype, q.get_device()
+    ok = dtype in _DTYPES
+    for t in tensors:
+        ok = ok and t.is_cuda and t.get_device() == index and t.dtype == dtype and (
+            not require_contiguous or t.is_contiguous())
+    if not ok:
         raise ValueError("Inputs must be contiguous BF16 (or FP16) on one CUDA device")
-    if torch.cuda.get_device_capability(q.device)[0] != 10:
+    if _major(index) != 10:
         raise ValueError("This implementation is written for SM100/Blackwell")
     return rotary
+
+
+def _query_mode(q, k, v, gq, gk, cos, sin, kn, out, causal, hf, eps, scale, variant):
+    """Row-prepare of K and the attention kernel in one C call (the second starts as a dependent of the first)."""
+    b, hq, s, d = q.shape
+    index = q.get_device()
+    with _on_device(index):
+        _call(_lib.load().kf_optimized_attention(
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), gq.data_ptr(), gk.data_ptr(), _ptr(cos), _ptr(sin), kn.data_ptr(),
+            out.data_ptr(), b, hq, k.shape[1], s, d, _DTYPES[q.dtype], 1 if causal else 0, 1 if hf else 0, eps,
+            d ** -0.5 if scale is None else scale, *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(kn),
+            *_strides3(out), status_word(q.device).data_ptr(), variant or _default_variant(), _raw_stream(index)))
 
 
 def optimized_attention(q, k, v, gq, gk, cos=None, sin=None, *, causal=False,
@@ -184,26 +221,23 @@ def optimized_attention(q, k, v, gq, gk, cos=None, sin=None, *, causal=False,
     _validate(q, k, v, gq, gk, cos, sin, mode, bn, norm_style)
     if not (eps > 0):
         raise ValueError("eps must be positive")
-    out = torch.empty_like(q) if out is None else out
-    kn = torch.empty_like(k) if kn is None else kn
-    if out.shape != q.shape or out.dtype != q.dtype or kn.shape != k.shape or kn.dtype != k.dtype:
+    if out is None:
+        out = torch.empty_like(q)
+    elif out.shape != q.shape or out.dtype != q.dtype:
         raise ValueError("out / kn must match q / k in shape and dtype")
-    with torch.cuda.device(q.device):
-        if mode == "unfused":
+    if kn is None:
+        kn = torch.empty_like(k)
+    elif kn.shape != k.shape or kn.dtype != k.dtype:
+        raise ValueError("out / kn must match q / k in shape and dtype")
+    if mode == "unfused":
+        with torch.cuda.device(q.device):
             prepare_rows(k, gk, cos, sin, norm_style=norm_style, eps=eps, out=kn)
             qn = prepare_rows(q, gq, cos, sin, norm_style=norm_style, eps=eps)
             attention_forward(qn, kn, v, gq, cos, sin, out, causal=causal, norm_style=norm_style,
                               fuse_q=False, eps=eps, scale=scale, variant=variant)
-        else:
-            # one C call for both launches
-            b, hq, s, d = q.shape
-            sc = float(d ** -0.5 if scale is None else scale)
-            _call(_lib.load().kf_optimized_attention(
-                _ptr(q), _ptr(k), _ptr(v), _ptr(gq), _ptr(gk), _ptr(cos), _ptr(sin), _ptr(kn), _ptr(out),
-                b, hq, k.shape[1], s, d, _DTYPES[q.dtype], int(bool(causal)), int(norm_style == "hf"), float(eps), sc,
-                *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(kn), *_strides3(out),
-                status_word(q.device).data_ptr(), int(variant) if variant else _default_variant(),
-                torch.cuda.current_stream().cuda_stream))
+    else:
+        _query_mode(q, k, v, gq, gk, cos, sin, kn, out, causal, norm_style == "hf", float(eps),
+                    None if scale is None else float(scale), int(variant) if variant else 0)
     return out
 
 
@@ -247,14 +281,7 @@ def launch_attention(inputs, out, *, causal=False, mode="query", bm=64, bn=64, w
         prepare_rows(k, gk, cos, sin, norm_style=style, out=kn)
         prepare_rows(q, gq, cos, sin, norm_style=style, out=qn)
         return attention_forward(qn, kn, v, gq, cos, sin, out, causal=causal, norm_style=style, fuse_q=False)
-    # both launches in one C call (the attention kernel then starts as a dependent of the prepare)
-    b, hq, s, d = q.shape
-    with torch.cuda.device(q.device):
-        _call(_lib.load().kf_optimized_attention(
-            _ptr(q), _ptr(k), _ptr(v), _ptr(gq), _ptr(gk), _ptr(cos), _ptr(sin), _ptr(kn), _ptr(out),
-            b, hq, k.shape[1], s, d, _DTYPES[q.dtype], int(bool(causal)), int(bool(hf_norm)), 1e-6, float(d ** -0.5),
-            *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(kn), *_strides3(out),
-            status_word(q.device).data_ptr(), _default_variant(), torch.cuda.current_stream().cuda_stream))
+    _query_mode(q, k, v, gq, gk, cos, sin, kn, out, causal, hf_norm, 1e-6, None, 0)
     return out
 
 
@@ -292,14 +319,8 @@ def fused(q, k, v, gq, gk, cos, sin, causal, eps=1e-6, scale=None, norm_style="q
         flat = out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
     kn = torch.empty(k.shape, dtype=k.dtype, device=k.device)
     gq, gk = gq.contiguous(), gk.contiguous()
-    sc = float(d ** -0.5 if scale is None else scale)
-    with torch.cuda.device(q.device):
-        # both launches in one C call (the attention kernel then starts as a dependent of the prepare)
-        _call(_lib.load().kf_optimized_attention(
-            _ptr(q), _ptr(k), _ptr(v), _ptr(gq), _ptr(gk), _ptr(cos), _ptr(sin), _ptr(kn), _ptr(out),
-            b, hq, k.shape[1], s, d, _DTYPES[q.dtype], int(bool(causal)), int(style == "hf"), float(eps), sc,
-            *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(kn), *_strides3(out),
-            status_word(q.device).data_ptr(), _default_variant(), torch.cuda.current_stream().cuda_stream))
+    _query_mode(q, k, v, gq, gk, cos, sin, kn, out, causal, style == "hf", float(eps),
+                None if scale is None else float(scale), 0)
     return flat
 
 
@@ -323,14 +344,13 @@ def factored_attention(q, k, v, gq, gk, *, causal=False, eps=1e-6, scale=None, o
         raise ValueError("out / kn must match q / k in shape and dtype")
     b, hq, s, d = q.shape
     sc = float(d ** -0.5 if scale is None else scale)
-    with torch.cuda.device(q.device):
-        st = status_word(q.device)
-        stream = torch.cuda.current_stream().cuda_stream
+    index = q.get_device()
+    with _on_device(index):
         _call(lib.kf_factored_attention(
             _ptr(q), _ptr(k), _ptr(v), _ptr(gq), _ptr(gk), _ptr(kn), _ptr(out),
             b, hq, k.shape[1], s, d, _DTYPES[q.dtype], int(bool(causal)), float(eps), sc,
             *_strides3(q), *_strides3(k), *_strides3(v), *_strides3(kn), *_strides3(out),
-            st.data_ptr(), int(variant), stream))
+            status_word(q.device).data_ptr(), int(variant), _raw_stream(index)))
     return out
 
 

@@ -67,6 +67,19 @@ cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     return launch_kernel_ex(kern, grid, block, smem, st, false, std::forward<Args>(args)...);
 }
 
+// Let a kernel use `bytes` of dynamic shared memory: set at its first launch on each device (0.6 us a call).
+template <auto KERN> cudaError_t allow_smem(int bytes) {
+    static std::atomic<unsigned long long> done{0};  // bit d: set on device d (two threads may both set it)
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
+    if (bit & done.load(std::memory_order_acquire)) return cudaSuccess;
+    e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 // Element stride of a dimension of extent n: a multiple of 8 (16 bytes), positive unless the dimension has a
 // single entry.  A zero stride over n > 1 entries (an expanded / broadcast view) is refused: the TMA maps
@@ -185,9 +198,9 @@ template <int D, typename T, bool FACTORED = false> int launch_prepare(const kf:
 template <int D, typename T>
 int launch_attn_basic(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                       const kf::AttnArgs& a, cudaStream_t st) {
-    auto kern = kf::attn_fwd_basic_kernel<D, T>;
+    constexpr auto kern = kf::attn_fwd_basic_kernel<D, T>;
     constexpr int smem = kf::attn_basic_smem_bytes<D>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
     const long long n_mblk = (a.S + kf::kBM - 1) / kf::kBM;
     const long long grid = n_mblk * a.B * a.Hq;
@@ -200,8 +213,8 @@ int launch_attn_basic(const CUtensorMap& mq, const CUtensorMap& mk, const CUtens
 template <typename T, bool FACTORED = false>
 int launch_attn_ws(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                    const kf::AttnArgs& a, cudaStream_t st) {
-    auto kern = kf::attn_fwd_ws_kernel<T, FACTORED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (FACTORED ? kf::kWsSmemBytesFactored : kf::kWsSmemBytes));
+    constexpr auto kern = kf::attn_fwd_ws_kernel<T, FACTORED>;
+    cudaError_t e = allow_smem<kern>((FACTORED ? kf::kWsSmemBytesFactored : kf::kWsSmemBytes));
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
     const int G = a.Hq / a.Hkv;
     const long long n_mblk = (a.S + kf::kBM - 1) / kf::kBM;
@@ -217,9 +230,9 @@ int launch_attn_ws(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
 template <int D, typename T, bool FACTORED = false>
 int launch_attn_ws1(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                     const kf::AttnArgs& a, cudaStream_t st, bool dependent = false) {
-    auto kern = kf::attn_fwd_ws1_kernel<D, T, FACTORED>;
+    constexpr auto kern = kf::attn_fwd_ws1_kernel<D, T, FACTORED>;
     constexpr int smem = kf::ws1_smem_bytes<D>(FACTORED);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
     const long long n_mblk = (a.S + kf::kBM - 1) / kf::kBM;
     const long long grid = n_mblk * a.B * a.Hq;
@@ -294,8 +307,8 @@ int sched_slot(unsigned int** out) {
 template <typename T>
 int launch_attn_persist(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                         const kf::AttnArgs& a0, cudaStream_t st, bool dependent = false) {
-    auto kern = kf::attn_fwd_persist_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kf::kPsSmemBytes);
+    constexpr auto kern = kf::attn_fwd_persist_kernel<T>;
+    cudaError_t e = allow_smem<kern>(kf::kPsSmemBytes);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
     kf::AttnArgs a = a0;
     if (int r = sched_slot(&a.sched)) return r;
@@ -314,8 +327,8 @@ int launch_attn_persist(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
 template <typename T>
 int launch_attn_persist256(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kf::AttnArgs& a0,
                            cudaStream_t st, bool dependent = false) {
-    auto kern = kf::attn_fwd_persist256_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kf::kP2SmemBytes);
+    constexpr auto kern = kf::attn_fwd_persist256_kernel<T>;
+    cudaError_t e = allow_smem<kern>(kf::kP2SmemBytes);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
     kf::AttnArgs a = a0;
     if (int r = sched_slot(&a.sched)) return r;
@@ -332,8 +345,8 @@ int launch_attn_persist256(const CUtensorMap& mq, const CUtensorMap& mk, const C
 template <typename T>
 int launch_attn_pair256(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kf::AttnArgs& a0,
                         cudaStream_t st, bool dependent = false) {
-    auto kern = kf::attn_fwd_pair256_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kf::kPrSmemBytes);
+    constexpr auto kern = kf::attn_fwd_pair256_kernel<T>;
+    cudaError_t e = allow_smem<kern>(kf::kPrSmemBytes);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
     kf::AttnArgs a = a0;
     if (int r = sched_slot(&a.sched)) return r;
