@@ -198,9 +198,9 @@ attn_fwd_persist256_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 if (!mbar_wait_abortable(c->s_full + buf, (gg >> 1) & 1, s_abort)) { fail = kStatusP2SFull; break; }
                 tc_fence_after();
                 const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= it.m0);
-                if (!plain || !softmax_ordinary<T, false>(lane_base + col_sb, cs, rs)) {
+                if (!plain || !softmax_ordinary<T, kPolyPairsOneTile, false>(lane_base + col_sb, cs, rs)) {
                     const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                    rs = softmax_general<D, T>(lane_base + col_sb, lane_base + kColO, cs, lim, rs, jj > 0 ? c->pv_done + ((gg - 1) & 1) : nullptr,
+                    rs = softmax_general<D, T, kPolyPairsOneTile>(lane_base + col_sb, lane_base + kColO, cs, lim, rs, jj > 0 ? c->pv_done + ((gg - 1) & 1) : nullptr,
                                                ((gg - 1) >> 1) & 1, s_abort);
                     if (!rs.ok) { fail = kStatusP2PvDone; break; }
                 }

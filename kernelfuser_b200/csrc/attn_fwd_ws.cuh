@@ -134,11 +134,12 @@ __device__ __forceinline__ void exp2_poly2(float x0, float x1, float& p0, float&
     p1 = __int_as_float(__float_as_int(q1) + (__float_as_int(r1) << 23));
 }
 
-// Which pairs of a 32-pair sub-block row go through the polynomial (the rest use MUFU ex2).
-#ifndef KF_POLY_MASK
-#define KF_POLY_MASK 0x88888888u  // every 4th pair: 25 %
-#endif
-constexpr uint32_t kPolyPairMask = KF_POLY_MASK;
+// Which pairs of a 32-pair sub-block row go through the polynomial (the rest use MUFU ex2).  MUFU takes 8 clocks of a
+// scheduler per element, a polynomial pair ~17 issue clocks; where the line lies best depends on what else issues.
+// B200, 8 of 32 evenly spaced -> these: 7 in the kernels of one tile per CTA or CTA pair B=1 S=16384 2025 -> 1982 us, 8-GPU shard
+// of B=16 S=4096 309 -> 305, D=256 B=8 S=8192 3575 -> 3527; the two-tile kernels want 8 (2291 -> 2268 us on B=16 S=4096;
+// with 6 or 7 2335 to 2359).
+constexpr uint32_t kPolyPairsOneTile = 0x84210842u, kPolyPairsTwoTile = 0x88844888u;
 
 // ---- softmax of one 64-key sub-block of one row
 // A row's exponent base is the maximum of its first sub-block and from then on of each one with a score more than
@@ -152,7 +153,7 @@ struct RowSoftmax {
 };
 
 // Probabilities of the row's 64 scores against base m, packed into pk; returns their sum.
-template <typename T>
+template <typename T, uint32_t POLY>
 __device__ __forceinline__ float exp_sub_block(const uint32_t (&sr)[2][32], float c, float m, uint32_t (&pk)[32]) {
     const f32x2 c2 = f2_pack(c, c), nm2 = f2_pack(-m, -m);
     f32x2 psum = f2_pack(0.f, 0.f);
@@ -161,7 +162,7 @@ __device__ __forceinline__ float exp_sub_block(const uint32_t (&sr)[2][32], floa
         const float u0 = __uint_as_float(sr[i / 16][2 * (i % 16)]), u1 = __uint_as_float(sr[i / 16][2 * (i % 16) + 1]);
         float x0, x1, p0, p1;
         f2_unpack(f2_fma(f2_pack(u0, u1), c2, nm2), x0, x1);
-        if ((kPolyPairMask >> i) & 1u) {
+        if ((POLY >> i) & 1u) {
             exp2_poly2(x0, x1, p0, p1);
         } else {
             p0 = fast_exp2(x0);
@@ -195,7 +196,7 @@ template <int D> __device__ __forceinline__ void rescale_output(uint32_t taddr, 
 // Not inlined: these are few of a long row's sub-blocks, and the loop of the others has to stay one short straight run of
 // code.  B200, against the same kernels with mask, maximum and rescale inside the loop (2 s of back-to-back calls):
 // B=16 S=4096 32/8 heads 2358 -> 2320 us, B=1 S=16384 2049 -> 2015 us, B=4 S=2048 193.4 -> 190.8 us.
-template <int D, typename T>
+template <int D, typename T, uint32_t POLY>
 __device__ __noinline__ RowSoftmax softmax_general(uint32_t taddr, uint32_t taddr_o, float c, int lim, RowSoftmax rs,
                                                    uint64_t* prev_pv, uint32_t parity, volatile int* abort_flag) {
     uint32_t sr[2][32], pk[32];
@@ -216,7 +217,7 @@ __device__ __noinline__ RowSoftmax softmax_general(uint32_t taddr, uint32_t tadd
         alpha = fast_exp2(rs.m - m_blk);  // 0 on the first sub-block
         rs.m = m_blk;
     }
-    const float sum = exp_sub_block<T>(sr, c, rs.m, pk);
+    const float sum = exp_sub_block<T, POLY>(sr, c, rs.m, pk);
     tmem_st32(taddr, pk);  // P overwrites its S
     rs.den = rs.den * alpha + sum;
     if (prev_pv != nullptr && __any_sync(0xffffffffu, grow)) {
@@ -233,20 +234,20 @@ __device__ __noinline__ RowSoftmax softmax_general(uint32_t taddr, uint32_t tadd
 // nothing stored, when a score of the warp lies too far above it.  The exponentials do not depend on the maximum, so
 // the two chains overlap.  MAX_FIRST orders the source for the compiler: with two softmax warps per scheduler (D = 128)
 // the maximum first is 2-5 % of a launch faster, with one (D = 256) the exponentials first by 3 %.
-template <typename T, bool MAX_FIRST>
+template <typename T, uint32_t POLY, bool MAX_FIRST>
 __device__ __forceinline__ bool softmax_ordinary(uint32_t taddr, float c, RowSoftmax& rs) {
     uint32_t sr[2][32], pk[32];
     tmem_ld32(taddr, sr[0]);
     tmem_ld32(taddr + 32, sr[1]);
     tmem_wait_ld();
     float sum = 0.f;
-    if (!MAX_FIRST) sum = exp_sub_block<T>(sr, c, rs.m, pk);
+    if (!MAX_FIRST) sum = exp_sub_block<T, POLY>(sr, c, rs.m, pk);
     float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
     for (int i = 0; i < 64; i += 2)
         mx[(i / 2) & 3] = max3(mx[(i / 2) & 3], __uint_as_float(sr[i / 32][i % 32]), __uint_as_float(sr[i / 32][i % 32 + 1]));
     if (__any_sync(0xffffffffu, fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * c > rs.m + kGrowLimit)) return false;
-    if (MAX_FIRST) sum = exp_sub_block<T>(sr, c, rs.m, pk);
+    if (MAX_FIRST) sum = exp_sub_block<T, POLY>(sr, c, rs.m, pk);
     tmem_st32(taddr, pk);  // P overwrites its S
     rs.den += sum;
     return true;
@@ -409,9 +410,9 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                     !mbar_wait_abortable(s_full + 2 * t + buf, (jj >> 1) & 1, s_abort)) { fail = kStatusWsSFull; break; }
                 tc_fence_after();
                 const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= tl.m0);
-                if (!plain || !softmax_ordinary<T, true>(lane_base + col_sb, c, rs)) {
+                if (!plain || !softmax_ordinary<T, kPolyPairsTwoTile, true>(lane_base + col_sb, c, rs)) {
                     const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                    rs = softmax_general<D, T>(lane_base + col_sb, lane_base + col_o, c, lim, rs, jj > 0 ? pv_done + 2 * t + ((jj - 1) & 1) : nullptr,
+                    rs = softmax_general<D, T, kPolyPairsTwoTile>(lane_base + col_sb, lane_base + col_o, c, lim, rs, jj > 0 ? pv_done + 2 * t + ((jj - 1) & 1) : nullptr,
                                                ((jj - 1) >> 1) & 1, s_abort);
                     if (!rs.ok) { fail = kStatusWsPvDone; break; }
                 }

@@ -64,10 +64,13 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     constexpr uint32_t kIdescQK = umma_idesc(Num<T>::kFmt, 0, kBM, kSub);
     constexpr uint32_t kIdescPV = umma_idesc(Num<T>::kFmt, 1, kBM, D);
 
-    // An earlier CTA or launch failed: drain quickly.  One thread reads the word and the whole CTA follows that
-    // reading, so no warp can leave while others go on to barriers the leaver would have served.
+    // An earlier CTA or launch may have failed.  One thread reads the word now and looks at it after the set-up (its
+    // ~500 clocks from L2 then overlap the barriers, the raw Q copy and the TMEM allocation: 1-3 % of a launch of short
+    // rows), and the whole CTA follows that reading, so no warp can leave while others go on to barriers the
+    // leaver would have served.
     KF_W1_STAMP(0);
-    if (__syncthreads_or(threadIdx.x == 0 && *reinterpret_cast<volatile int*>(a.status) != 0)) return;
+    int status = 0;
+    if (threadIdx.x == 0) status = *reinterpret_cast<volatile int*>(a.status);
     KF_W1_STAMP(1);
 
     extern __shared__ uint8_t smem_raw[];
@@ -90,6 +93,7 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     uint64_t* pv_done = bars + 18;  // [jj & 1]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
     volatile int* s_abort = reinterpret_cast<volatile int*>(bars + 21);
+    volatile int* s_dead = s_abort + 1;
     [[maybe_unused]] float* s_inv = reinterpret_cast<float*>(bars + 64);  // [row] inverse RMS of the raw Q rows (factored form)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -131,6 +135,8 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         mbar_expect_tx(q_full, kW256QBytes);
 #pragma unroll
         for (int bx = 0; bx < NB; ++bx) tma_load_4d(smem_q + bx * kBoxBytes, &tm_q, q_full, bx * 64, m0, h, b);
+        *s_dead = status;
+        if (status != 0) *s_abort = 1;  // (the exit then waits for the raw Q tile)
     }
     if (warp == 0) {
         __syncwarp();
@@ -146,7 +152,9 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     int fail = 0;
     int kv_issued = 0;  // producer bookkeeping for the exit path
 
-    if (warp < 4) {
+    if (*s_dead != 0) {
+        // an earlier launch or CTA failed: fall through to the common exit
+    } else if (warp < 4) {
         // =================================================== softmax, Q prologue, epilogue
         const int r = tid;
         const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
@@ -208,9 +216,9 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             tc_fence_after();
             if (jj == 0) KF_W1_STAMP(4);
             const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= m0);
-            if (!plain || !softmax_ordinary<T, D == 128>(lane_base + col_sb, c, rs)) {
+            if (!plain || !softmax_ordinary<T, kPolyPairsOneTile, D == 128>(lane_base + col_sb, c, rs)) {
                 const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                rs = softmax_general<D, T>(lane_base + col_sb, lane_base + kColO, c, lim, rs, jj > 0 ? pv_done + ((jj - 1) & 1) : nullptr,
+                rs = softmax_general<D, T, kPolyPairsOneTile>(lane_base + col_sb, lane_base + kColO, c, lim, rs, jj > 0 ? pv_done + ((jj - 1) & 1) : nullptr,
                                            ((jj - 1) >> 1) & 1, s_abort);
                 if (!rs.ok) { fail = kStatusWsPvDone; break; }
             }
