@@ -78,14 +78,15 @@ int kf_prepare_rows(const void* x, void* y, const void* gamma, const void* cos_t
  * variant: 0 = choose automatically.  D = 128: kernel 3 when the launch has
  * at least 8192 query tiles (B*Hq*ceil(S/128)) and 2048 < S < 8192, else
  * kernel 5 (factored form: kernel 2 above 8192 tiles, else 5).  D = 256:
- * kernel 3 when the launch holds at least 200 sub-blocks of 64 keys per SM,
- * else kernel 2.
+ * kernel 3 when the launch holds at least 200 sub-blocks of 64 keys per SM (85
+ * with Hq/Hkv even and two work items per pair of SMs), else kernel 2.
  * 1 = baseline kernel (softmax and MMA serialised inside a CTA; any head dim),
  * 2 = pipelined, warp-specialised kernel, one launch per work item (D = 128:
  * two Q tiles per CTA; D = 256: one),
  * 3 = persistent form of kernel 2: one CTA per SM takes work items from a
  * device counter and prepares the next item's Q while the running one
- * computes (D = 128 and D = 256; same results as kernel 2 bit for bit),
+ * computes (D = 128 and D = 256; same results as kernel 2 bit for bit).  At
+ * D = 256 with Hq/Hkv even a pair of SMs works on two heads together.
  * 5 = the one-tile-per-CTA kernel of D = 256 instantiated for D = 128 with
  * two CTAs per SM: faster than 2 and 3 on small problems, slower on large
  * ones.  4 is not used. */

@@ -34,18 +34,17 @@ constexpr int kPrItemRing = 8;
 constexpr int kPrSmemBytes = kP2QBytes + kPrRing * kPrStageBytes + 1024 + kPsCtrlBytes;
 static_assert(kPrSmemBytes <= 232448, "shared memory of an SM");
 
-// Pair item `idx` in (batch, KV head)-major order, heaviest query block first within a group; `rank` picks the head.
+// Pair item `idx` in the order of sg_decode (see ps_decode); `rank` picks the head.
 __device__ __forceinline__ P2Item pr_decode(int idx, uint32_t rank, const AttnArgs& a) {
     P2Item it;
     const int G = a.Hq / a.Hkv, pairs = G / 2;
     const int n_mblk = (a.S + kBM - 1) / kBM;
     const int n_sub_all = (a.S + kSub - 1) / kSub;
-    const int upg = n_mblk * pairs;
-    const int grp = idx / upg, r = idx % upg;
-    it.b = grp / a.Hkv;
-    it.kh = grp % a.Hkv;
-    it.m0 = (n_mblk - 1 - r / pairs) * kBM;
-    it.h = it.kh * G + 2 * (r % pairs) + static_cast<int>(rank);
+    const SgItem sg = sg_decode(idx, a.B * a.Hkv, a.sg_groups, a.sg_first, n_mblk, pairs);
+    it.b = sg.grp / a.Hkv;
+    it.kh = sg.grp % a.Hkv;
+    it.m0 = (n_mblk - 1 - sg.level) * kBM;
+    it.h = it.kh * G + 2 * sg.sub + static_cast<int>(rank);
     it.nsub = a.causal ? min((it.m0 + kBM) / kSub, n_sub_all) : n_sub_all;
     return it;
 }

@@ -50,18 +50,17 @@ struct P2Item {
     int b, h, kh, m0, nsub;
 };
 
-// Tile `idx` in (batch, KV head)-major order, heaviest query block first within a group.
+// Tile `idx` in the order of sg_decode (see ps_decode).
 __device__ __forceinline__ P2Item p2_decode(int idx, const AttnArgs& a) {
     P2Item it;
     const int G = a.Hq / a.Hkv;
     const int n_mblk = (a.S + kBM - 1) / kBM;
     const int n_sub_all = (a.S + kSub - 1) / kSub;
-    const int upg = n_mblk * G;
-    const int grp = idx / upg, r = idx % upg;
-    it.b = grp / a.Hkv;
-    it.kh = grp % a.Hkv;
-    it.m0 = (n_mblk - 1 - r / G) * kBM;
-    it.h = it.kh * G + r % G;
+    const SgItem sg = sg_decode(idx, a.B * a.Hkv, a.sg_groups, a.sg_first, n_mblk, G);
+    it.b = sg.grp / a.Hkv;
+    it.kh = sg.grp % a.Hkv;
+    it.m0 = (n_mblk - 1 - sg.level) * kBM;
+    it.h = it.kh * G + sg.sub;
     it.nsub = a.causal ? min((it.m0 + kBM) / kSub, n_sub_all) : n_sub_all;
     return it;
 }

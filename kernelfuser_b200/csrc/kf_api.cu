@@ -260,8 +260,10 @@ constexpr long long kDependentMaxTiles = KF_DEPENDENT_MAX_TILES;
 #define KF_DEPENDENT_PERSIST 1
 #endif
 
-// Sub-blocks of work per SM from which variant 0 picks the persistent kernel at D = 256.
+// Sub-blocks of work per SM from which variant 0 picks the persistent kernel at D = 256: whatever else holds, and on
+// SM pairs with two items for each.
 constexpr long long kPersist256MinSubBlocksPerSm = 200;
+constexpr long long kPair256MinSubBlocksPerSm = 85;
 
 // Variant 0 at D = 128 picks the persistent two-tile kernel from this many 128-row query tiles, for sequence
 // lengths strictly between the two limits below, and the one-tile-per-CTA kernel everywhere else.
@@ -465,12 +467,25 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
         if (factored) variant = tiles > kAutoPersistMinTiles ? 2 : 5;
         else variant = (tiles >= kAutoPersistMinTiles && mid) ? 3 : 5;
     }
-    if (D == 128 && variant == 3) {
-        CUtensorMap mk64, mv64;  // the persistent kernel streams K/V in 64-row tiles
-        if (int r = make_map(&mk64, kn, dtype, B, Hkv, S, D, k_sb, k_sh, k_ss, 64)) return r;
-        if (int r = make_map(&mv64, v, dtype, B, Hkv, S, D, v_sb, v_sh, v_ss, 64)) return r;
-        return dtype == KF_BF16 ? launch_attn_persist<__nv_bfloat16>(mq, mk64, mv64, mo, a, st, dependent && KF_DEPENDENT_PERSIST)
-                                : launch_attn_persist<__half>(mq, mk64, mv64, mo, a, st, dependent && KF_DEPENDENT_PERSIST);
+    // Query heads that share a KV head in even numbers run the persistent form of D = 256 on SM pairs.
+    const bool on_pairs = D == 256 && !factored && (Hq / Hkv) % 2 == 0;
+    if (D == 256 && variant == 0 && !factored) {
+        // The persistent kernels hide a tile's fixed costs (raw Q copy, transform, copy into TMEM, output store) behind
+        // the previous / next tile's main loop, and a pair streams half the K and V; they pay once every SM has enough
+        // 64-key sub-blocks to work through and a pair has items to choose from.  B200, one launch item per tile ->
+        // SM pairs, by sub-blocks per SM and items per pair:
+        //   446, 3.5 (B=1 S=16384, 4/2 heads)   473 -> 437 us     62, 6.9 (B=8 S=1024, 16/8)  150 -> 165
+        //   228, 6.9 (B=2 S=4096, 16/8)         315 -> 275        65, 2.6 (B=1 S=3072, 16/8)  101 ->  95
+        //   117, 6.9 (B=4 S=2048, 16/8)         209 -> 192        59, 3.5 (B=4 S=2048, 8/4)   106 -> 105
+        //   114, 3.5 (B=1 S=4096, 16/8)         159 -> 152       112, 1.7 (B=1 S=8192, 4/2)   127 -> 129
+        //    88, 3.0 (B=1 S=3500, 16/8)         129 -> 119        77, 1.4 (B=1 S=6700, 4/2)    98 -> 101
+        // The form of one CTA per tile (odd numbers) pays from about 200 (B=8 S=8192: -11 %; +4 ... +18 % at a hundred).
+        const long long n_mblk = (S + kf::kBM - 1) / kf::kBM, n_sub_all = (S + kf::kSub - 1) / kf::kSub;
+        const long long per_head = causal ? n_mblk * (n_mblk + 1) : n_mblk * n_sub_all;
+        const long long work = (long long)B * Hq * per_head, sms = sm_count();
+        if (work >= kPersist256MinSubBlocksPerSm * sms ||
+            (on_pairs && work >= kPair256MinSubBlocksPerSm * sms && (long long)B * Hq * n_mblk >= 2 * sms))
+            variant = 3;
     }
     {
         // CTA order (sg_decode).  Small launches - up to about ten CTAs per resident slot - interleave all
@@ -481,10 +496,14 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
         const long long groups = (long long)B * Hkv;
         const long long n_mblk = (S + kf::kBM - 1) / kf::kBM;
         const int G = Hq / Hkv;
-        long long ctas_per_group = n_mblk * G;  // one 128-row tile per CTA
-        long long slots = sm_count();           // CTAs resident at a time
+        long long ctas_per_group = n_mblk * G;  // work items of a group: one 128-row tile each
+        long long slots = sm_count();           // items in work at a time
         if (D == 128 && variant == 5) slots *= 2;
-        // (the two-tiles-per-CTA kernel of D = 128 only serves large launches and keeps the group-major order)
+        // (the two-tile kernels of D = 128 only serve large launches and keep the group-major order)
+        if (on_pairs && variant == 3) {  // two tiles per SM pair
+            ctas_per_group /= 2;
+            slots /= 2;
+        }
         long long fit = kSuperGroupBytes / (2LL * S * D * 2);  // K and V of one group, bytes
         if (fit < 1) fit = 1;
         a.sg_groups = 1;
@@ -504,6 +523,13 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
             }
         }
     }
+    if (D == 128 && variant == 3) {
+        CUtensorMap mk64, mv64;  // the persistent kernel streams K/V in 64-row tiles
+        if (int r = make_map(&mk64, kn, dtype, B, Hkv, S, D, k_sb, k_sh, k_ss, 64)) return r;
+        if (int r = make_map(&mv64, v, dtype, B, Hkv, S, D, v_sb, v_sh, v_ss, 64)) return r;
+        return dtype == KF_BF16 ? launch_attn_persist<__nv_bfloat16>(mq, mk64, mv64, mo, a, st, dependent && KF_DEPENDENT_PERSIST)
+                                : launch_attn_persist<__half>(mq, mk64, mv64, mo, a, st, dependent && KF_DEPENDENT_PERSIST);
+    }
     if (D == 128 && variant == 5) {
         CUtensorMap mk64, mv64;  // K/V stream in 64-row tiles
         if (int r = make_map(&mk64, kn, dtype, B, Hkv, S, D, k_sb, k_sh, k_ss, 64)) return r;
@@ -521,19 +547,7 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
         return dtype == KF_BF16 ? launch_attn_ws<__nv_bfloat16>(mq, mk, mv, mo, a, st)
                                 : launch_attn_ws<__half>(mq, mk, mv, mo, a, st);
     }
-    if (D == 256 && variant == 0 && !factored) {
-        // The persistent kernel hides a tile's fixed costs (raw Q copy, transform, copy into TMEM, output store)
-        // behind the previous / next tile's main loop; it pays once every SM has a few hundred 64-key sub-blocks
-        // to work through (B200, one launch item per tile -> SM pairs: B=8 S=8192 16/8 heads 4222 -> 3502 us, B=1 S=16384
-        // 4/2 heads 473 -> 437; with about a hundred sub-blocks per SM the one-tile kernel balances better: B=1 S=4096
-        // 155 -> 165, B=4 S=1024 82 -> 102).
-        const long long n_mblk = (S + kf::kBM - 1) / kf::kBM, n_sub_all = (S + kf::kSub - 1) / kf::kSub;
-        const long long per_head = causal ? n_mblk * (n_mblk + 1) : n_mblk * n_sub_all;
-        if ((long long)B * Hq * per_head >= kPersist256MinSubBlocksPerSm * sm_count()) variant = 3;
-    }
-    if (D == 256 && variant == 3 && !factored && (Hq / Hkv) % 2 == 0) {
-        // Query heads that share a KV head in even numbers run on SM pairs, 7-13 % faster than one CTA per tile
-        // wherever the persistent form is chosen at all.
+    if (on_pairs && variant == 3) {
         CUtensorMap mk32, mv64;  // each CTA of a pair loads 32 keys of K and half of the columns of V
         if (int r = make_map(&mk32, kn, dtype, B, Hkv, S, D, k_sb, k_sh, k_ss, 32)) return r;
         if (int r = make_map(&mv64, v, dtype, B, Hkv, S, D, v_sb, v_sh, v_ss, 64)) return r;
