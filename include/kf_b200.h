@@ -75,9 +75,10 @@ int kf_prepare_rows(const void* x, void* y, const void* gamma, const void* cos_t
  * fuse_q = 0: q is already prepared (mode 'unfused').
  * kn is the prepared K from kf_prepare_rows; v is the raw V.
  * scale is the softmax scale (the reference passes D^-0.5).
- * variant: 0 = choose automatically.  D = 128: kernel 3 when the launch has
- * at least 8192 query tiles (B*Hq*ceil(S/128)) and 2048 < S < 8192, else
- * kernel 5 (factored form: kernel 2 above 8192 tiles, else 5).  D = 256:
+ * variant: 0 = choose automatically.  D = 128: kernel 3 for S > 2048 when the
+ * launch holds at least 2000 sub-blocks of 64 keys per SM (Hq/Hkv even) or at
+ * least 8192 query tiles (B*Hq*ceil(S/128)) with S < 8192, else kernel 5
+ * (factored form: kernel 2 above 8192 tiles, else 5).  D = 256:
  * kernel 3 when the launch holds at least 200 sub-blocks of 64 keys per SM (85
  * with Hq/Hkv even and two work items per pair of SMs), else kernel 2.
  * 1 = baseline kernel (softmax and MMA serialised inside a CTA; any head dim),

@@ -265,8 +265,10 @@ constexpr long long kDependentMaxTiles = KF_DEPENDENT_MAX_TILES;
 constexpr long long kPersist256MinSubBlocksPerSm = 200;
 constexpr long long kPair256MinSubBlocksPerSm = 85;
 
-// Variant 0 at D = 128 picks the persistent two-tile kernel from this many 128-row query tiles, for sequence
-// lengths strictly between the two limits below, and the one-tile-per-CTA kernel everywhere else.
+// Variant 0 at D = 128 picks the persistent two-tile kernel for sequences longer than kAutoPersistMinS: from
+// kAutoPersistMinSubBlocksPerSm sub-blocks of work per SM where a work item is two heads of a KV head, else from
+// kAutoPersistMinTiles query tiles below kAutoPersistMaxS; the one-tile-per-CTA kernel serves everything else.
+constexpr long long kAutoPersistMinSubBlocksPerSm = 2000;
 constexpr long long kAutoPersistMinTiles = 8192;
 constexpr int kAutoPersistMinS = 2048, kAutoPersistMaxS = 8192;
 
@@ -454,18 +456,25 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
         return fail(KF_EINVAL, "the factored form runs on kernels 0, 2 and 5 only");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool dependent = after_prepare && (long long)B * Hq * ((S + kf::kBM - 1) / kf::kBM) <= kDependentMaxTiles;
-    // Automatic choice at D = 128.  The one-tile-per-CTA kernel (two CTAs per SM, groups interleaved heaviest
-    // first) fills the SMs, keeps the causal tail short and has the better steady state (two independent CTAs
-    // instead of two tiles in step): measured on B200 it is 3-9 % faster than the persistent two-tile kernel at
-    // S <= 2048 and S >= 8192 whatever the size of the launch, and 1-17 % faster on launches below about eight
-    // thousand query tiles.  In between (S = 3072 ... 6144 with at least 8192 tiles, C4 and its 2-GPU shard among
-    // them) the persistent kernel wins by 2-6 %: it hides the per-tile fixed costs, which weigh most there, and
-    // its tile pair shares one K/V stream.  (The factored form exists for kernels 2 and 5 only.)
+    // Automatic choice at D = 128.  The one-tile-per-CTA kernel (two CTAs per SM, groups interleaved heaviest first)
+    // fills the SMs, keeps the causal tail short and takes fewest clocks per sub-block; the persistent kernel hides the
+    // per-tile fixed costs and its tile pair shares one K/V stream, which also saves power: long launches run at the
+    // 1 kW limit and then at a higher clock (1.51 against 1.45 GHz).  B200, one-tile -> persistent, back to back (in
+    // brackets: alone), by sub-blocks per SM, 32/8 heads unless said:
+    //   3570 B=1 S=16384  1999 -> 1974 us (1738 -> 1712)      2013 B=1 S=12288  1149 -> 1147 ( 984 ->  990)
+    //   3597 B=4 S=8192   2149 -> 2092    (1856 -> 1821)      1827 B=8 S=4096   1208 -> 1185 (1031 -> 1021)
+    //   3542 B=8 S=4096 without mask 2097 -> 2037             1771 B=1 S=8192 without mask 995 -> 1002 (847 -> 864)
+    //   2034 B=4 S=6144   1264 -> 1230    (1077 -> 1066)       913 B=4 S=4096    608 ->  608 ( 518 ->  536)
+    //   2075 B=16 S=3072  1459 -> 1454    (1247 -> 1253)
+    // and 717 -> 824 at B=16 S=2048.  (The factored form exists for kernels 2 and 5 only.)
     if (D == 128 && variant == 0) {
-        const long long tiles = (long long)B * Hq * ((S + kf::kBM - 1) / kf::kBM);
-        const bool mid = S > kAutoPersistMinS && S < kAutoPersistMaxS;
+        const long long n_mblk = (S + kf::kBM - 1) / kf::kBM, n_sub_all = (S + kf::kSub - 1) / kf::kSub;
+        const long long tiles = (long long)B * Hq * n_mblk;
+        const long long work = (long long)B * Hq * (causal ? n_mblk * (n_mblk + 1) : n_mblk * n_sub_all);
+        const bool two_heads = (Hq / Hkv) % 2 == 0 && S > kAutoPersistMinS && work >= kAutoPersistMinSubBlocksPerSm * sm_count();
+        const bool mid = tiles >= kAutoPersistMinTiles && S > kAutoPersistMinS && S < kAutoPersistMaxS;
         if (factored) variant = tiles > kAutoPersistMinTiles ? 2 : 5;
-        else variant = (tiles >= kAutoPersistMinTiles && mid) ? 3 : 5;
+        else variant = two_heads || mid ? 3 : 5;
     }
     // Query heads that share a KV head in even numbers run the persistent form of D = 256 on SM pairs.
     const bool on_pairs = D == 256 && !factored && (Hq / Hkv) % 2 == 0;
