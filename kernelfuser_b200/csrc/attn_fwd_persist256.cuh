@@ -1,4 +1,5 @@
-// Persistent, warp-specialised tcgen05 flash-attention forward kernel for head dim 256.
+// Persistent, warp-specialised tcgen05 flash-attention forward kernel for head dim 256, one CTA per tile: serves odd numbers
+// of query heads per KV head (even ones run on SM pairs, attn_fwd_pair256.cuh).
 //
 // Same operator and the same inner pipeline as the D = 256 instantiation of attn_fwd_ws256.cuh (reference:
 // `attention_v2_kernel`, src/e1_rope_publication_v1.py:609-649; Q prologue :619-623; rounding contract `_rows`
