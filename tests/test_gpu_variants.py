@@ -105,3 +105,21 @@ def test_d256_sm_pairs_match_oracle(b, s, hq, hkv, causal, dtype):
     kf.check_status()
     m = orc.metric(out.cpu(), ref)
     assert orc.within_tolerance(m), (b, s, hq, hkv, m)
+
+
+@pytest.mark.parametrize("variant", [2, 3])
+def test_d256_kernels_drain_on_a_status(variant):
+    # a launch that finds an earlier failure leaves without touching the output; on SM pairs both CTAs follow one reading
+    xs = [x.cuda() for x in kf.make_inputs(2, 300, 4, 2, 256, theta=1e4, seed=68)]
+    word = kf.status_word(xs[0].device)
+    word.fill_(7)
+    out = torch.full_like(xs[0], float("nan"))
+    kf.optimized_attention(*xs, causal=True, out=out, variant=variant)
+    torch.cuda.synchronize()
+    with pytest.raises(kf.KernelStatusError, match="7"):
+        kf.check_status()
+    assert torch.isnan(out).all()
+    again = kf.optimized_attention(*xs, causal=True, out=out, variant=variant)
+    torch.cuda.synchronize()
+    kf.check_status()
+    assert torch.isfinite(again).all()
