@@ -14,10 +14,11 @@
 // B200, one CTA per tile -> pairs (back-to-back calls): B=8 S=8192 16/8 heads 3988 -> 3502 us, its 8-GPU shard 509 -> 472,
 // B=1 S=16384 4/2 heads 466 -> 437.
 //
-// Barriers.  What the issuer waits for lives in CTA 0 and takes arrivals of both CTAs (remote arrivals with
-// cluster scope); what it signals - tcgen05.commit with both CTAs' mask - arrives at the same offset in both.
-// Copies are plain per-CTA TMA loads on the CTA's own barrier; CTA 1's otherwise idle issuer warp relays "my half
-// has landed" to CTA 0.  Work items are claimed by CTA 0's scheduler and published to both CTAs.
+// Barriers.  What the issuer waits for lives in CTA 0, takes arrivals of both CTAs and is waited for with cluster
+// scope; what it signals - tcgen05.commit with both CTAs' mask - arrives at the same offset in both.  Copies are plain
+// per-CTA TMA loads on the CTA's own barrier; CTA 1's otherwise idle issuer warp sees its half land and relays that to
+// CTA 0 with a release: the issuer never looks at CTA 1's own barrier, so the release and its own acquire are what orders
+// the copy before the MMA that reads it.  Work items are claimed by CTA 0's scheduler and published to both CTAs.
 #pragma once
 #include "attn_fwd_persist256.cuh"
 
@@ -76,6 +77,7 @@ struct PrCtrl {
 };
 static_assert(sizeof(PrCtrl) <= kPsCtrlBytes, "control block too large");
 
+// Bounded, abortable wait on a barrier that the other CTA arrives on.
 __device__ __forceinline__ bool pr_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
     const long long t0 = clock64();
@@ -392,7 +394,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     const int tiles = 2 * pr_decode(idx, rank, a).nsub;
                     for (int i = 0; i < tiles; ++i) {
                         if (!mbar_wait_abortable(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; break; }
-                        remote_arrive_relaxed(full0 + 8 * st);
+                        remote_arrive(full0 + 8 * st);  // passes on shared memory that CTA 0's MMAs read
                         if (++st == kPrRing) { st = 0; par ^= 1; }
                     }
                 }
@@ -428,7 +430,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 uint32_t nq = 0, np = 0;
                 // scores of sub-block j of the running tile; the tile's last one also reports "every Q K^T done"
                 auto take_k = [&](bool last) {
-                    if (!mbar_wait_abortable(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; return; }
+                    if (!pr_wait(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; return; }
                     tc_fence_after();
                     issue_qk(st, nq & 1);
                     umma_commit_pair(c->s_full + (nq & 1));
@@ -441,7 +443,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     const int idx = pr_take_item(c, n, fail);
                     if (idx < 0) break;
                     const P2Item it = pr_decode(idx, rank, a);
-                    if (!mbar_wait_abortable(&c->q_ready, n & 1, s_abort)) { fail = kStatusP2QReady; break; }
+                    if (!pr_wait(&c->q_ready, n & 1, s_abort)) { fail = kStatusP2QReady; break; }
                     take_k(it.nsub == 1);
                     for (int jj = 0; jj < it.nsub && !fail; ++jj) {
                         if (jj + 1 < it.nsub) {
@@ -449,10 +451,10 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                             if (fail) break;
                         }
                         // ---- O += P V of sub-block jj
-                        if (!mbar_wait_abortable(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; break; }
+                        if (!pr_wait(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; break; }
                         // the first P V of a tile overwrites the previous tile's output: the epilogue must have read it
-                        if (jj == 0 && n > 0 && !mbar_wait_abortable(&c->o_free, (n - 1) & 1, s_abort)) { fail = kStatusP2OFree; break; }
-                        if (!mbar_wait_abortable(c->p_ready + (np & 1), (np >> 1) & 1, s_abort)) { fail = kStatusP2PReady; break; }
+                        if (jj == 0 && n > 0 && !pr_wait(&c->o_free, (n - 1) & 1, s_abort)) { fail = kStatusP2OFree; break; }
+                        if (!pr_wait(c->p_ready + (np & 1), (np >> 1) & 1, s_abort)) { fail = kStatusP2PReady; break; }
                         tc_fence_after();
                         issue_pv(st, np & 1, jj > 0 ? 1u : 0u);
                         umma_commit_pair(c->pv_done + (np & 1));

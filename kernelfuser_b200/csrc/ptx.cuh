@@ -104,9 +104,10 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ void remote_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// The same where nothing written to memory is handed over: tensor-memory accesses are ordered by tcgen05.wait and
-// tcgen05.fence, copies by their own barrier.  A release at cluster scope first waits for the thread's earlier
-// accesses, which in the score hand-over of every sub-block cost a third of the kernel's time.
+// The same where only tensor memory is handed over: its accesses are ordered by tcgen05.wait and tcgen05.fence.  (Not
+// for shared memory, however it was written: an arrival that passes on "the copy has landed" is a release.)  A release
+// at cluster scope first waits for the thread's earlier accesses; in the score hand-over of every sub-block the kernel
+// took half as long again with it.
 __device__ __forceinline__ void remote_arrive_relaxed(uint32_t bar) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
