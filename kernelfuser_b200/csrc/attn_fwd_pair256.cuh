@@ -61,6 +61,7 @@ struct PrCtrl {
     uint64_t s_full[2];          // [buffer]
     uint64_t pv_done[2];         // [g & 1]
     uint64_t qk_done;            // every Q K^T of the tile has completed (the Q columns may be overwritten)
+    uint64_t mma_done;           // every MMA of the launch has completed
     // within a CTA
     uint64_t q_full;             // raw Q of the next tile is in the Q buffer
     uint64_t q_free;             // Q group (4): the Q buffer has been copied out and may be refilled
@@ -130,6 +131,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         mbar_init(&c->q_ready, 8);
         mbar_init(&c->q_free, 4);
         mbar_init(&c->qk_done, 1);
+        mbar_init(&c->mma_done, 1);
         mbar_init(&c->o_free, 8);
         mbar_init(&c->den_full, 4);
         mbar_init(&c->den_free, 4);
@@ -168,6 +170,20 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         *s_abort = 1;
         remote_store(map_to_cta(&c->abort_flag, rank ^ 1u), 1);
         atomicCAS(a.status, 0, code);
+    };
+
+    // Last step of warp 9 in both CTAs: the asynchronous MMAs and the arrivals of their commits end before either CTA frees
+    // its TMEM or leaves.  `tiles` ring stages of `items` items have been consumed; a launch that gives up waits for
+    // the MMAs that were issued only.  (Every wait is bounded.)
+    auto drain_mma = [&](int items, int tiles, bool failed) {
+        mbar_wait(&c->mma_done, 0);
+        if (failed) return;
+        for (int i = 0; i < kPrRing; ++i)
+            if (tiles > i) mbar_wait_abortable(c->kv_empty + i, ((tiles - 1 - i) / kPrRing) & 1, s_abort);
+        const int last = tiles / 2 - 1;  // last sub-block
+        mbar_wait_abortable(c->pv_done + (last & 1), (last >> 1) & 1, s_abort);
+        if (last > 0) mbar_wait_abortable(c->pv_done + ((last - 1) & 1), ((last - 1) >> 1) & 1, s_abort);
+        mbar_wait_abortable(&c->qk_done, (items - 1) & 1, s_abort);
     };
 
     int fail = 0;
@@ -388,10 +404,12 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 const uint32_t full0 = map_to_cta(c->kv_full, 0);
                 int st = 0;
                 uint32_t par = 0;
-                for (int n = 0; !fail; ++n) {
+                int n = 0, total = 0;
+                for (; !fail; ++n) {
                     const int idx = pr_take_item(c, n, fail);
                     if (idx < 0) break;
                     const int tiles = 2 * pr_decode(idx, rank, a).nsub;
+                    total += tiles;
                     for (int i = 0; i < tiles; ++i) {
                         if (!mbar_wait_abortable(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; break; }
                         remote_arrive(full0 + 8 * st);  // passes on shared memory that CTA 0's MMAs read
@@ -399,6 +417,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     }
                 }
                 if (fail) give_up(fail);
+                drain_mma(n, total, fail != 0);
             }
         } else if (warp == 9) {
             // ============================================ MMA issuer of the pair
@@ -439,7 +458,8 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     if (last) umma_commit_pair(&c->qk_done);
                     if (++st == kPrRing) { st = 0; par ^= 1; }
                 };
-                for (int n = 0; !fail; ++n) {
+                int n = 0;
+                for (; !fail; ++n) {
                     const int idx = pr_take_item(c, n, fail);
                     if (idx < 0) break;
                     const P2Item it = pr_decode(idx, rank, a);
@@ -464,6 +484,10 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     }
                 }
                 if (fail) give_up(fail);
+                if (nq > 0) {  // (else nothing was issued; CTA 1's wait then runs out)
+                    umma_commit_pair(&c->mma_done);
+                    drain_mma(n, static_cast<int>(nq + np), fail != 0);
+                }
             }
         } else if (warp == 10) {
             // ============================================ scheduler (CTA 0) and raw-Q producer
@@ -512,7 +536,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         if (warp == 10 && elect_one() && q_issued > 0) mbar_wait(&c->q_full, (q_issued - 1) & 1);
     }
     __syncthreads();
-    cluster_sync();  // no MMA, commit or remote arrival of the pair is under way any more
+    cluster_sync();  // both CTAs have drained the MMAs and their commits, and no thread sends a remote arrival any more
     if (warp == 0) tmem_dealloc_pair(tmem_base, kTmemCols);
     // The last CTA to leave resets the work counter for the next launch that uses it.
     if (tid == 0) {

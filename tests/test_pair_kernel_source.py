@@ -26,3 +26,15 @@ def test_issuer_waits_with_cluster_scope_where_the_other_cta_arrives():
     waits = re.findall(r"!(\w+)\(&?c->(\w+)", issuer)
     assert {n for _, n in waits} == {n for n, _ in arrivals()} - {"item_full"}
     assert {f for f, _ in waits} == {"pr_wait"}
+
+
+def test_every_commit_is_awaited_in_both_ctas_before_they_leave():
+    committed = set(re.findall(r"umma_commit_pair\(&?c->(\w+)", CODE))
+    drain = CODE[CODE.index("auto drain_mma"):CODE.index("int fail = 0;")]
+    awaited = set(re.findall(r"mbar_wait(?:_abortable)?\(&?c->(\w+)", drain))
+    # (the softmax warps wait for every s_full: their row sums need each sub-block's scores)
+    assert committed - {"s_full"} == awaited
+    # called by the issuer of CTA 0 and by the relay of CTA 1, the last commit being the one of every MMA
+    assert len(re.findall(r"\bdrain_mma\(", CODE)) == 2
+    assert re.search(r"umma_commit_pair\(&c->mma_done\);\s*drain_mma\(", CODE)
+    assert CODE.rindex("drain_mma(") < CODE.rindex("tmem_dealloc_pair(")
