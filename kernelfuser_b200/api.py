@@ -73,9 +73,11 @@ def _strides3(t: torch.Tensor):
     return t.stride()[:3]
 
 
-# Raw handle of the current stream of a device index: what torch.cuda.current_stream(i).cuda_stream returns, without
-# the Stream object built around it (0.1 against 3.3 us).
-_raw_stream = torch._C._cuda_getCurrentRawStream
+# Two bindings that torch's own generated code calls, without the objects that the public functions build around them (the
+# stream handle: 0.1 against 3.3 us).  They are private names: a torch build without them takes the public functions.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 _capability_major = {}  # device index -> compute capability, major
 
 
@@ -91,7 +93,7 @@ _HERE = nullcontext()
 
 def _on_device(index: int):
     """Context in which device ``index`` is current: nothing to do in the usual case that it is already."""
-    return _HERE if torch._C._cuda_getDevice() == index else torch.cuda.device(index)
+    return _HERE if _current_device() == index else torch.cuda.device(index)
 
 
 def _ptr(t):
