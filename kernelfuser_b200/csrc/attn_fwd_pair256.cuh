@@ -10,15 +10,16 @@
 // of them pull that from L2 together (~1550 clocks per sub-block where the MMAs take 1024).  A pair copies every K/V
 // tile once for 256 rows - each CTA loads 32 of the 64 keys of K and half of the columns of V - so the stream halves,
 // and the ring holds five sub-blocks instead of two and a half.  What is left is the chain P V, Q K^T, hand-over,
-// softmax of a score buffer (~1350 clocks per sub-block); large launches run at the 1 kW power limit.
-// B200, one CTA per tile -> pairs (back-to-back calls): B=8 S=8192 16/8 heads 3988 -> 3502 us, its 8-GPU shard 509 -> 472,
-// B=1 S=16384 4/2 heads 466 -> 437.
+// softmax of a score buffer; large launches run at the 1 kW power limit.
+// B200, one CTA per tile -> pairs (back-to-back calls): B=8 S=8192 16/8 heads 3988 -> 3178 us, its 8-GPU shard 509 -> 408.
 //
-// Barriers.  What the issuer waits for lives in CTA 0, takes arrivals of both CTAs and is waited for with cluster
-// scope; what it signals - tcgen05.commit with both CTAs' mask - arrives at the same offset in both.  Copies are plain
-// per-CTA TMA loads on the CTA's own barrier; CTA 1's otherwise idle issuer warp sees its half land and relays that to
-// CTA 0 with a release: the issuer never looks at CTA 1's own barrier, so the release and its own acquire are what orders
-// the copy before the MMA that reads it.  Work items are claimed by CTA 0's scheduler and published to both CTAs.
+// Barriers.  What the issuer waits for lives in CTA 0; what it signals - tcgen05.commit with both CTAs' mask - arrives at
+// the same offset in both.  A K/V stage is full when the halves of both CTAs have landed: each CTA announces its half
+// on CTA 0's barrier and its TMA copy (.cta_group::2, into its own shared memory) completes there, so the barrier that the
+// issuer waits on is that of the copies themselves.  (With a relay in CTA 1 that waits for its copy and tells CTA 0
+// in a release that CTA 0 acquires at cluster scope, B=8 S=8192 16/8 heads took 4750-4900 us against 3178.)  Tensor
+// memory is handed over with relaxed arrivals: tcgen05.wait and tcgen05.fence order its accesses.  Work items are claimed
+// by CTA 0's scheduler and published to both CTAs.
 #pragma once
 #include "attn_fwd_persist256.cuh"
 
@@ -55,7 +56,7 @@ struct PrCtrl {
     uint64_t q_ready;            // 8 Q-group warps: the tile's prepared Q is in TMEM
     uint64_t o_free;             // 8 Q-group warps: the finished tile's output has been read
     uint64_t p_ready[2];         // [buffer] 8 softmax warps
-    uint64_t kv_full[kPrRing];   // own copy (1 arrival + bytes); in CTA 0 also CTA 1's relay
+    uint64_t kv_full[kPrRing];   // both CTAs' halves (1 arrival + bytes each)
     // signalled by the issuer's commits, in both CTAs
     uint64_t kv_empty[kPrRing];
     uint64_t s_full[2];          // [buffer]
@@ -73,12 +74,12 @@ struct PrCtrl {
     int abort_flag;
     int item[kPrItemRing];
     int dead;
-    int pad[1];
+    int issued[2];               // CTA 0: K/V copies that each CTA has issued
     float den[kBM];
 };
 static_assert(sizeof(PrCtrl) <= kPsCtrlBytes, "control block too large");
 
-// Bounded, abortable wait on a barrier that the other CTA arrives on.
+// Bounded, abortable wait that also sees what the other CTA released.
 __device__ __forceinline__ bool pr_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     if (mbar_try_wait_cluster(bar, parity)) return true;
     const long long t0 = clock64();
@@ -144,7 +145,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         }
 #pragma unroll
         for (int i = 0; i < kPrRing; ++i) {
-            mbar_init(c->kv_full + i, leader ? 2 : 1);
+            mbar_init(c->kv_full + i, 2);
             mbar_init(c->kv_empty + i, 1);
         }
 #pragma unroll
@@ -172,7 +173,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         atomicCAS(a.status, 0, code);
     };
 
-    // Last step of warp 9 in both CTAs: the asynchronous MMAs and the arrivals of their commits end before either CTA frees
+    // Last step of the issuer and of CTA 1's producer: the asynchronous MMAs and the arrivals of their commits end before either CTA frees
     // its TMEM or leaves.  `tiles` ring stages of `items` items have been consumed; a launch that gives up waits for
     // the MMAs that were issued only.  (Every wait is bounded.)
     auto drain_mma = [&](int items, int tiles, bool failed) {
@@ -361,10 +362,11 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 int s = 0;            // ring stage of the next tile
                 uint32_t epar = 1;    // parity to wait for on the stage's empty barrier (passes at once on the first turn)
                 const int r0 = static_cast<int>(rank);
+                const uint32_t full0 = map_to_cta(c->kv_full, 0);
                 // next tile of the consumption order, this CTA's half of it
                 auto next_stage = [&]() -> uint8_t* {
                     if (!mbar_wait_abortable(c->kv_empty + s, epar, s_abort)) { fail = kStatusP2KvEmpty; return nullptr; }
-                    mbar_expect_tx(c->kv_full + s, kPrStageBytes);
+                    remote_expect_tx(full0 + 8 * s, kPrStageBytes);
                     ++kv_issued;
                     return smem_kv + s * kPrStageBytes;
                 };
@@ -373,7 +375,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     if (dst == nullptr) return;
 #pragma unroll
                     for (int bx = 0; bx < NB; ++bx)
-                        tma_load_4d(dst + bx * kPrKBoxBytes, &tm_k, c->kv_full + s, bx * 64, j * kSub + r0 * (kSub / 2), it.kh, it.b);
+                        tma_load_4d_pair(dst + bx * kPrKBoxBytes, &tm_k, full0 + 8 * s, bx * 64, j * kSub + r0 * (kSub / 2), it.kh, it.b);
                     if (++s == kPrRing) { s = 0; epar ^= 1; }
                 };
                 auto emit_v = [&](int j, const P2Item& it) {  // all 64 keys, half of the columns
@@ -381,12 +383,13 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     if (dst == nullptr) return;
 #pragma unroll
                     for (int bx = 0; bx < NB / 2; ++bx)
-                        tma_load_4d(dst + bx * kPrVBoxBytes, &tm_v, c->kv_full + s, r0 * (D / 2) + bx * 64, j * kSub, it.kh, it.b);
+                        tma_load_4d_pair(dst + bx * kPrVBoxBytes, &tm_v, full0 + 8 * s, r0 * (D / 2) + bx * 64, j * kSub, it.kh, it.b);
                     if (++s == kPrRing) { s = 0; epar ^= 1; }
                 };
                 // (see attn_fwd_persist.cuh: the first K copy waits for the row-prepare this grid may depend on)
                 grid_dep_wait();
-                for (int n = 0; !fail; ++n) {
+                int n = 0;
+                for (; !fail; ++n) {
                     const int idx = pr_take_item(c, n, fail);
                     if (idx < 0) break;
                     const P2Item it = pr_decode(idx, rank, a);
@@ -397,29 +400,10 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     }
                 }
                 if (fail) give_up(fail);
+                if (!leader) drain_mma(n, kv_issued, fail != 0);
+                remote_store(map_to_cta(c->issued + rank, 0), kv_issued);
             }
-        } else if (warp == 9 && !leader) {
-            // ============================================ relay: this CTA's half of a stage has landed -> CTA 0
-            if (elect_one()) {
-                const uint32_t full0 = map_to_cta(c->kv_full, 0);
-                int st = 0;
-                uint32_t par = 0;
-                int n = 0, total = 0;
-                for (; !fail; ++n) {
-                    const int idx = pr_take_item(c, n, fail);
-                    if (idx < 0) break;
-                    const int tiles = 2 * pr_decode(idx, rank, a).nsub;
-                    total += tiles;
-                    for (int i = 0; i < tiles; ++i) {
-                        if (!mbar_wait_abortable(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; break; }
-                        remote_arrive(full0 + 8 * st);  // passes on shared memory that CTA 0's MMAs read
-                        if (++st == kPrRing) { st = 0; par ^= 1; }
-                    }
-                }
-                if (fail) give_up(fail);
-                drain_mma(n, total, fail != 0);
-            }
-        } else if (warp == 9) {
+        } else if (warp == 9 && leader) {
             // ============================================ MMA issuer of the pair
             if (elect_one()) {
                 const uint32_t kv_addr = smem_u32(smem_kv);
@@ -449,7 +433,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 uint32_t nq = 0, np = 0;
                 // scores of sub-block j of the running tile; the tile's last one also reports "every Q K^T done"
                 auto take_k = [&](bool last) {
-                    if (!pr_wait(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; return; }
+                    if (!mbar_wait_abortable(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; return; }
                     tc_fence_after();
                     issue_qk(st, nq & 1);
                     umma_commit_pair(c->s_full + (nq & 1));
@@ -463,7 +447,7 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     const int idx = pr_take_item(c, n, fail);
                     if (idx < 0) break;
                     const P2Item it = pr_decode(idx, rank, a);
-                    if (!pr_wait(&c->q_ready, n & 1, s_abort)) { fail = kStatusP2QReady; break; }
+                    if (!mbar_wait_abortable(&c->q_ready, n & 1, s_abort)) { fail = kStatusP2QReady; break; }
                     take_k(it.nsub == 1);
                     for (int jj = 0; jj < it.nsub && !fail; ++jj) {
                         if (jj + 1 < it.nsub) {
@@ -471,10 +455,10 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                             if (fail) break;
                         }
                         // ---- O += P V of sub-block jj
-                        if (!pr_wait(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; break; }
+                        if (!mbar_wait_abortable(c->kv_full + st, par, s_abort)) { fail = kStatusP2KvFull; break; }
                         // the first P V of a tile overwrites the previous tile's output: the epilogue must have read it
-                        if (jj == 0 && n > 0 && !pr_wait(&c->o_free, (n - 1) & 1, s_abort)) { fail = kStatusP2OFree; break; }
-                        if (!pr_wait(c->p_ready + (np & 1), (np >> 1) & 1, s_abort)) { fail = kStatusP2PReady; break; }
+                        if (jj == 0 && n > 0 && !mbar_wait_abortable(&c->o_free, (n - 1) & 1, s_abort)) { fail = kStatusP2OFree; break; }
+                        if (!mbar_wait_abortable(c->p_ready + (np & 1), (np >> 1) & 1, s_abort)) { fail = kStatusP2PReady; break; }
                         tc_fence_after();
                         issue_pv(st, np & 1, jj > 0 ? 1u : 0u);
                         umma_commit_pair(c->pv_done + (np & 1));
@@ -524,19 +508,21 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     // ---- common exit
     __syncwarp();
     tc_fence_before();
-    __syncthreads();
+    cluster_sync();  // every role of both CTAs has ended (and a failure of either shows in both)
     if (!dead && *s_abort != 0) {
-        // leave no copy in flight into this CTA's shared memory (CTA 0's barriers may miss the other CTA's arrival for
-        // a stage; the wait then runs out after far longer than a copy takes)
-        if (warp == 8 && elect_one()) {
-#pragma unroll
-            for (int s = 0; s < kPrRing; ++s)
-                if (kv_issued > s) mbar_wait(c->kv_full + s, ((kv_issued - 1 - s) / kPrRing) & 1);
+        // Leave no copy in flight.  Both CTAs' K/V copies complete on CTA 0's barriers: arrivals that a CTA did not make
+        // are made up for, so that every phase ends with the copies that were issued.
+        if (leader && warp == 8 && elect_one()) {
+            volatile int* issued = c->issued;
+            const int lo = min(issued[0], issued[1]), hi = max(issued[0], issued[1]);
+            for (int i = lo; i < hi; ++i) mbar_arrive(c->kv_full + i % kPrRing);
+            for (int i = 0; i < kPrRing; ++i)
+                if (hi > i) mbar_wait(c->kv_full + i, ((hi - 1 - i) / kPrRing) & 1);
         }
         if (warp == 10 && elect_one() && q_issued > 0) mbar_wait(&c->q_full, (q_issued - 1) & 1);
     }
     __syncthreads();
-    cluster_sync();  // both CTAs have drained the MMAs and their commits, and no thread sends a remote arrival any more
+    cluster_sync();  // no copy, MMA, commit or remote arrival of the pair is under way any more
     if (warp == 0) tmem_dealloc_pair(tmem_base, kTmemCols);
     // The last CTA to leave resets the work counter for the next launch that uses it.
     if (tid == 0) {

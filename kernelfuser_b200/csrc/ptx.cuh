@@ -104,10 +104,14 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ void remote_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// The same where only tensor memory is handed over: its accesses are ordered by tcgen05.wait and tcgen05.fence.  (Not
-// for shared memory, however it was written: an arrival that passes on "the copy has landed" is a release.)  A release
-// at cluster scope first waits for the thread's earlier accesses; in the score hand-over of every sub-block the kernel
-// took half as long again with it.
+// Arrival that announces bytes to come; hands over nothing itself.
+__device__ __forceinline__ void remote_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                 : "memory");
+}
+// remote_arrive where only tensor memory is handed over: its accesses are ordered by tcgen05.wait and tcgen05.fence.
+// (Not for shared memory.)  A release at cluster scope first waits for the thread's earlier accesses; in the score
+// hand-over of every sub-block the kernel took half as long again with it.
 __device__ __forceinline__ void remote_arrive_relaxed(uint32_t bar) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -144,6 +148,16 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* m, uin
         "[%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2),
         "r"(c3)
+        : "memory");
+}
+// The same for a CTA of an SM pair: the data lands in this CTA's shared memory, the completion on a barrier of either
+// CTA (`bar`: its cluster address, see map_to_cta).
+__device__ __forceinline__ void tma_load_4d_pair(void* dst, const CUtensorMap* m, uint32_t bar, int c0, int c1, int c2,
+                                                 int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
 // 4-D tiled store shared -> global (rows outside the tensor are clipped).

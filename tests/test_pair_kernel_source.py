@@ -18,14 +18,17 @@ def arrivals():
 
 def test_only_tensor_memory_is_handed_over_without_a_release():
     assert {n for n, relaxed in arrivals() if relaxed} == TENSOR_MEMORY
-    assert {n for n, relaxed in arrivals() if not relaxed} >= {"kv_full", "item_full"}
+    assert {n for n, relaxed in arrivals() if not relaxed} == {"item_full"}
 
 
-def test_issuer_waits_with_cluster_scope_where_the_other_cta_arrives():
-    issuer = RAW[RAW.index("MMA issuer of the pair"):RAW.index("scheduler (CTA 0)")]
-    waits = re.findall(r"!(\w+)\(&?c->(\w+)", issuer)
-    assert {n for _, n in waits} == {n for n, _ in arrivals()} - {"item_full"}
-    assert {f for f, _ in waits} == {"pr_wait"}
+def test_both_halves_of_a_stage_complete_on_the_barrier_that_the_issuer_waits_on():
+    # K and V of both CTAs are read by MMAs that CTA 0 issues: a copy that completed on CTA 1's own barrier would need
+    # a relay, and nothing but a release and an acquire at cluster scope would order it before the read
+    assert re.search(r"full0 = map_to_cta\(c->kv_full, 0\);", CODE)
+    copies = re.findall(r"(tma_load_4d\w*)\([^;]*?&tm_([kv]), ([^,]+),", CODE)
+    assert sorted(c[1] for c in copies) == ["k", "v"]
+    assert {(c[0], c[2]) for c in copies} == {("tma_load_4d_pair", "full0 + 8 * s")}
+    assert re.findall(r"(\w*expect_tx)\(([^,]*)", CODE) == [("remote_expect_tx", "full0 + 8 * s"), ("mbar_expect_tx", "&c->q_full")]
 
 
 def test_every_commit_is_awaited_in_both_ctas_before_they_leave():
@@ -34,7 +37,7 @@ def test_every_commit_is_awaited_in_both_ctas_before_they_leave():
     awaited = set(re.findall(r"mbar_wait(?:_abortable)?\(&?c->(\w+)", drain))
     # (the softmax warps wait for every s_full: their row sums need each sub-block's scores)
     assert committed - {"s_full"} == awaited
-    # called by the issuer of CTA 0 and by the relay of CTA 1, the last commit being the one of every MMA
+    # called by the issuer of CTA 0 and by the producer of CTA 1, the last commit being the one of every MMA
     assert len(re.findall(r"\bdrain_mma\(", CODE)) == 2
     assert re.search(r"umma_commit_pair\(&c->mma_done\);\s*drain_mma\(", CODE)
     assert CODE.rindex("drain_mma(") < CODE.rindex("tmem_dealloc_pair(")
