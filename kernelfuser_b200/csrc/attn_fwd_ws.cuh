@@ -80,9 +80,10 @@ __device__ __forceinline__ bool named_barrier_or(int id, int nthreads, bool pred
     return r != 0;
 }
 
+// Largest of three, NaN if one of them is.
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
 
@@ -145,6 +146,9 @@ constexpr uint32_t kPolyPairsOneTile = 0x84210842u, kPolyPairsTwoTile = 0x888448
 // A row's exponent base is the maximum of its first sub-block and from then on of each one with a score more than
 // kGrowLimit above the base, which keeps every probability at or below 2^8.  (Not rounded to a whole number: the
 // row's largest probability is then exactly 1, and in short rows its rounding is most of the error.)
+// A row with a NaN score, or a base that is not finite (a score of +inf, or nothing but -inf), comes out NaN: its
+// scores fail the comparison of an ordinary sub-block, and the general one makes the sum NaN.  The probabilities alone
+// would not show it everywhere: the polynomial's clamp turns a NaN into 2^-125.
 constexpr float kGrowLimit = 8.0f;  // log2 units
 struct RowSoftmax {
     float m = -INFINITY;  // exponent base (log2 units)
@@ -210,8 +214,8 @@ __device__ __noinline__ RowSoftmax softmax_general(uint32_t taddr, uint32_t tadd
         if (i + 1 >= lim) sr[i / 32][i % 32 + 1] = 0xff800000u;
         mx[(i / 2) & 1] = max3(mx[(i / 2) & 1], __uint_as_float(sr[i / 32][i % 32]), __uint_as_float(sr[i / 32][i % 32 + 1]));
     }
-    const float m_blk = fmaxf(mx[0], mx[1]) * c;
-    const bool grow = m_blk > rs.m + kGrowLimit;
+    const float m_blk = max3(mx[0], mx[1], mx[1]) * c;
+    const bool grow = !(m_blk <= rs.m + kGrowLimit);  // (or a NaN among the scores)
     float alpha = 1.f;
     if (grow) {
         alpha = fast_exp2(rs.m - m_blk);  // 0 on the first sub-block
@@ -219,7 +223,7 @@ __device__ __noinline__ RowSoftmax softmax_general(uint32_t taddr, uint32_t tadd
     }
     const float sum = exp_sub_block<T, POLY>(sr, c, rs.m, pk);
     tmem_st32(taddr, pk);  // P overwrites its S
-    rs.den = rs.den * alpha + sum;
+    rs.den = rs.den * alpha + sum + (rs.m - rs.m);  // (0, or NaN where the base is not finite)
     if (prev_pv != nullptr && __any_sync(0xffffffffu, grow)) {
         // O may only be touched once the previous P V has completed.  (pv_done alternates between two barriers, so a
         // phase cannot be lapped: the next P V needs this sub-block's P.)
@@ -246,7 +250,7 @@ __device__ __forceinline__ bool softmax_ordinary(uint32_t taddr, float c, RowSof
 #pragma unroll
     for (int i = 0; i < 64; i += 2)
         mx[(i / 2) & 3] = max3(mx[(i / 2) & 3], __uint_as_float(sr[i / 32][i % 32]), __uint_as_float(sr[i / 32][i % 32 + 1]));
-    if (__any_sync(0xffffffffu, fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]) * c > rs.m + kGrowLimit)) return false;
+    if (__any_sync(0xffffffffu, !(max3(max3(mx[0], mx[1], mx[2]), mx[3], mx[3]) * c <= rs.m + kGrowLimit))) return false;
     if (MAX_FIRST) sum = exp_sub_block<T, POLY>(sr, c, rs.m, pk);
     tmem_st32(taddr, pk);  // P overwrites its S
     rs.den += sum;
