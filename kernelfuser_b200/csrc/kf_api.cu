@@ -284,13 +284,31 @@ int sm_count() {
     return cached[dev];
 }
 
-// Work counters of the persistent kernel: {next item, CTAs that have left} per slot.  They live in the
-// library image (zero at load), the kernel's last CTA puts them back to zero, and launches take the slots in
-// turn, so that launches in flight on different streams of a device do not share one (up to kSchedSlots of them).
-constexpr int kSchedSlots = 64;
-__device__ unsigned int g_sched[kSchedSlots][2];
+// Work counters of the persistent kernels: {next item, CTAs that have left}, zero between launches (in the library image;
+// the last CTA of a launch puts them back).  Launches into a stream take the first kSchedSlots in turn, so two could only
+// share one if a launch were still running when that many later ones have been started.  A captured launch runs again
+// with every replay of its graph, next to whatever else is running: it gets one of the other kGraphSlots for itself,
+// which the graph, its clones and its executable forms own together and give back when the last of them is destroyed.
+constexpr int kSchedSlots = 1024, kGraphSlots = 1 << 14;
+__device__ unsigned int g_sched[kSchedSlots + kGraphSlots][2];
 
-int sched_slot(unsigned int** out) {
+std::atomic_flag g_slots_busy = ATOMIC_FLAG_INIT;  // guards the three below (plain data: graphs may outlive static objects)
+int g_slots_back[kGraphSlots], g_n_back, g_n_taken;  // slots given back; slots taken at least once
+
+int take_graph_slot() {  // -1: none left
+    while (g_slots_busy.test_and_set(std::memory_order_acquire)) {}
+    const int s = g_n_back > 0 ? g_slots_back[--g_n_back] : g_n_taken < kGraphSlots ? g_n_taken++ : -1;
+    g_slots_busy.clear(std::memory_order_release);
+    return s;
+}
+void CUDART_CB give_back_graph_slot(void* slot) {
+    while (g_slots_busy.test_and_set(std::memory_order_acquire)) {}
+    g_slots_back[g_n_back++] = static_cast<int>(reinterpret_cast<intptr_t>(slot));
+    g_slots_busy.clear(std::memory_order_release);
+}
+
+// The counters of the launch about to be made into `st`; NULL: it is being captured and every graph slot is taken.
+int sched_slot(cudaStream_t st, unsigned int** out) {
     static std::atomic<unsigned int*> base[64];
     static std::atomic<unsigned int> turn{0};
     int dev = 0;
@@ -304,18 +322,41 @@ int sched_slot(unsigned int** out) {
         bp = static_cast<unsigned int*>(p);
         base[dev].store(bp, std::memory_order_release);
     }
-    *out = bp + 2 * (turn.fetch_add(1, std::memory_order_relaxed) % kSchedSlots);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo_v2(st, &capture, nullptr, &graph, nullptr, nullptr) != cudaSuccess) {
+        cudaGetLastError();  // (the legacy stream next to a capture elsewhere: the launch itself reports that)
+        capture = cudaStreamCaptureStatusNone;
+    }
+    if (capture != cudaStreamCaptureStatusActive) {
+        *out = bp + 2 * (turn.fetch_add(1, std::memory_order_relaxed) % kSchedSlots);
+        return KF_OK;
+    }
+    *out = nullptr;
+    const int slot = take_graph_slot();
+    if (slot < 0) return KF_OK;
+    cudaUserObject_t owner = nullptr;
+    void* const tag = reinterpret_cast<void*>(static_cast<intptr_t>(slot));
+    cudaError_t e = cudaUserObjectCreate(&owner, tag, give_back_graph_slot, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        give_back_graph_slot(tag);
+        return fail(KF_ECUDA, "cudaUserObjectCreate failed: %s", cudaGetErrorString(e));
+    }
+    e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) {
+        cudaUserObjectRelease(owner, 1);  // (gives the slot back)
+        return fail(KF_ECUDA, "cudaGraphRetainUserObject failed: %s", cudaGetErrorString(e));
+    }
+    *out = bp + 2 * (kSchedSlots + slot);
     return KF_OK;
 }
 
 template <typename T>
 int launch_attn_persist(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
-                        const kf::AttnArgs& a0, cudaStream_t st, bool dependent = false) {
+                        const kf::AttnArgs& a, cudaStream_t st, bool dependent = false) {
     constexpr auto kern = kf::attn_fwd_persist_kernel<T>;
     cudaError_t e = allow_smem<kern>(kf::kPsSmemBytes);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
-    kf::AttnArgs a = a0;
-    if (int r = sched_slot(&a.sched)) return r;
     const int G = a.Hq / a.Hkv;
     const long long n_mblk = (a.S + kf::kBM - 1) / kf::kBM;
     const long long upg = (G % 2 == 0) ? n_mblk * (G / 2) : ((n_mblk + 1) / 2) * G;
@@ -329,13 +370,11 @@ int launch_attn_persist(const CUtensorMap& mq, const CUtensorMap& mk, const CUte
 }
 
 template <typename T>
-int launch_attn_persist256(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kf::AttnArgs& a0,
+int launch_attn_persist256(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kf::AttnArgs& a,
                            cudaStream_t st, bool dependent = false) {
     constexpr auto kern = kf::attn_fwd_persist256_kernel<T>;
     cudaError_t e = allow_smem<kern>(kf::kP2SmemBytes);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
-    kf::AttnArgs a = a0;
-    if (int r = sched_slot(&a.sched)) return r;
     const long long n_mblk = (a.S + kf::kBM - 1) / kf::kBM;
     const long long items = n_mblk * a.B * a.Hq;
     if (items > 0x7fffffffLL) return fail(KF_EINVAL, "too many tiles");
@@ -347,13 +386,11 @@ int launch_attn_persist256(const CUtensorMap& mq, const CUtensorMap& mk, const C
 }
 
 template <typename T>
-int launch_attn_pair256(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kf::AttnArgs& a0,
+int launch_attn_pair256(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const kf::AttnArgs& a,
                         cudaStream_t st, bool dependent = false) {
     constexpr auto kern = kf::attn_fwd_pair256_kernel<T>;
     cudaError_t e = allow_smem<kern>(kf::kPrSmemBytes);
     if (e != cudaSuccess) return fail(KF_ECUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
-    kf::AttnArgs a = a0;
-    if (int r = sched_slot(&a.sched)) return r;
     const long long n_mblk = (a.S + kf::kBM - 1) / kf::kBM;
     const long long items = n_mblk * a.B * (a.Hq / 2);
     if (items > 0x7fffffffLL) return fail(KF_EINVAL, "too many tiles");
@@ -495,6 +532,10 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
         if (work >= kPersist256MinSubBlocksPerSm * sms ||
             (on_pairs && work >= kPair256MinSubBlocksPerSm * sms && (long long)B * Hq * n_mblk >= 2 * sms))
             variant = 3;
+    }
+    if (variant == 3) {
+        if (int r = sched_slot(st, &a.sched)) return r;
+        if (a.sched == nullptr) variant = 2;  // same results without a counter, one launch item per CTA
     }
     {
         // CTA order (sg_decode).  Small launches - up to about ten CTAs per resident slot - interleave all

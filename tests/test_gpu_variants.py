@@ -65,9 +65,9 @@ def test_d256_variants_match_oracle(variant, s, hq, hkv, causal, dtype):
 
 
 def test_persistent_kernels_reuse_their_counter_slots():
-    # The persistent kernels take work from counters in the library image, 64 slots used in turn and reset by
-    # the last CTA of each launch: run more launches than slots, on two streams, both head dims, and compare
-    # every result with the first one of its kind.
+    # The persistent kernels take work from counters in the library image, slots used in turn and reset by the
+    # last CTA of each launch: run launches one behind the other on two streams, both head dims, more of them than
+    # there are slots, and compare every result with the first one of its kind.
     xs128 = [x.cuda() for x in kf.make_inputs(2, 640, 8, 2, 128, seed=5)]
     xs256 = [x.cuda() for x in kf.make_inputs(1, 512, 4, 2, 256, theta=1e4, seed=6)]
     ref128 = kf.optimized_attention(*xs128, causal=True, variant=3)
@@ -77,7 +77,7 @@ def test_persistent_kernels_reuse_their_counter_slots():
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     outs = []
-    for i in range(100):
+    for i in range(1100):
         xs, ref = (xs128, ref128) if i % 3 else (xs256, ref256)
         if i % 2:
             with torch.cuda.stream(side):
