@@ -67,17 +67,59 @@ cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t 
     return launch_kernel_ex(kern, grid, block, smem, st, false, std::forward<Args>(args)...);
 }
 
-// Let a kernel use `bytes` of dynamic shared memory: set at its first launch on each device (0.6 us a call).
+// Identity of the calling thread's CUDA context: never used again in a process, and a new one after a device reset.
+// 0: unknown (no context yet), to be treated as one never seen.
+unsigned long long context_id() {
+    using Fn = CUresult (*)(CUcontext, unsigned long long*);
+    static std::atomic<Fn> cached{nullptr};
+    Fn fn = cached.load(std::memory_order_acquire);
+    if (fn == nullptr) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            return 0;
+        fn = reinterpret_cast<Fn>(p);
+        cached.store(fn, std::memory_order_release);
+    }
+    unsigned long long id = 0;
+    return fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// Let a kernel use `bytes` of dynamic shared memory.  The setting belongs to the context: made at the kernel's first
+// launch in each (0.6 us).
 template <auto KERN> cudaError_t allow_smem(int bytes) {
-    static std::atomic<unsigned long long> done{0};  // bit d: set on device d (two threads may both set it)
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const unsigned long long bit = dev >= 0 && dev < 64 ? 1ull << dev : 0ull;
-    if (bit & done.load(std::memory_order_acquire)) return cudaSuccess;
-    e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    static std::atomic<unsigned long long> done[64];  // contexts by id (two threads may both set it)
+    const unsigned long long id = context_id();
+    if (id != 0 && done[id % 64].load(std::memory_order_acquire) == id) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done[id % 64].store(id, std::memory_order_release);
     return e;
+}
+
+// Device address, in the current context, of a variable of the library image; looked up once per context.
+struct SymbolCache {
+    std::atomic_flag busy = ATOMIC_FLAG_INIT;
+    unsigned long long id[64];
+    void* at[64];
+};
+cudaError_t symbol_address(SymbolCache& c, const void* symbol, void** out) {
+    const unsigned long long id = context_id();
+    const int i = static_cast<int>(id % 64);
+    auto locked = [&](auto&& body) {
+        while (c.busy.test_and_set(std::memory_order_acquire)) {}
+        body();
+        c.busy.clear(std::memory_order_release);
+    };
+    void* p = nullptr;
+    locked([&] { if (id != 0 && c.id[i] == id) p = c.at[i]; });
+    if (p == nullptr) {
+        cudaError_t e = cudaGetSymbolAddress(&p, symbol);
+        if (e != cudaSuccess) return e;
+        if (const unsigned long long now = context_id())  // (the call may have made the context)
+            locked([&] { c.id[now % 64] = now; c.at[now % 64] = p; });
+    }
+    *out = p;
+    return cudaSuccess;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -309,19 +351,12 @@ void CUDART_CB give_back_graph_slot(void* slot) {
 
 // The counters of the launch about to be made into `st`; NULL: it is being captured and every graph slot is taken.
 int sched_slot(cudaStream_t st, unsigned int** out) {
-    static std::atomic<unsigned int*> base[64];
+    static SymbolCache cache;
     static std::atomic<unsigned int> turn{0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return fail(KF_ECUDA, "cudaGetDevice failed");
-    unsigned int* bp = base[dev].load(std::memory_order_acquire);
-    if (bp == nullptr) {
-        void* p = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&p, g_sched);
-        if (e != cudaSuccess || p == nullptr)
-            return fail(KF_ECUDA, "cudaGetSymbolAddress(work counters) failed: %s", cudaGetErrorString(e));
-        bp = static_cast<unsigned int*>(p);
-        base[dev].store(bp, std::memory_order_release);
-    }
+    void* p = nullptr;
+    cudaError_t e = symbol_address(cache, g_sched, &p);
+    if (e != cudaSuccess) return fail(KF_ECUDA, "cudaGetSymbolAddress(work counters) failed: %s", cudaGetErrorString(e));
+    unsigned int* const bp = static_cast<unsigned int*>(p);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
     if (cudaStreamGetCaptureInfo_v2(st, &capture, nullptr, &graph, nullptr, nullptr) != cudaSuccess) {
@@ -337,7 +372,7 @@ int sched_slot(cudaStream_t st, unsigned int** out) {
     if (slot < 0) return KF_OK;
     cudaUserObject_t owner = nullptr;
     void* const tag = reinterpret_cast<void*>(static_cast<intptr_t>(slot));
-    cudaError_t e = cudaUserObjectCreate(&owner, tag, give_back_graph_slot, 1, cudaUserObjectNoDestructorSync);
+    e = cudaUserObjectCreate(&owner, tag, give_back_graph_slot, 1, cudaUserObjectNoDestructorSync);
     if (e != cudaSuccess) {
         give_back_graph_slot(tag);
         return fail(KF_ECUDA, "cudaUserObjectCreate failed: %s", cudaGetErrorString(e));
@@ -758,23 +793,11 @@ constexpr size_t kStaticScratchBytes = 32u << 20;  // 32 MiB: B*Hkv*S*D*2 bytes 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
 namespace {
-// The array's name is only a host-side handle; kernels need its device address,
-// which differs per device and is looked up once per device (with that device
-// current) through cudaGetSymbolAddress.
-std::atomic<void*> g_scratch_addr[64];  // (atomic: two host threads may make a device's first call at once)
-
+// The array's name is only a host-side handle; kernels need its device address.
 int static_scratch_for_current_device(void** out) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return fail(KF_ECUDA, "cudaGetDevice failed");
-    if (dev < 0 || dev >= 64) return fail(KF_ECUDA, "device ordinal %d out of range", dev);
-    void* p = g_scratch_addr[dev].load(std::memory_order_acquire);
-    if (p == nullptr) {
-        cudaError_t e = cudaGetSymbolAddress(&p, g_static_scratch);
-        if (e != cudaSuccess || p == nullptr)
-            return fail(KF_ECUDA, "cudaGetSymbolAddress(static scratch) failed: %s", cudaGetErrorString(e));
-        g_scratch_addr[dev].store(p, std::memory_order_release);  // (a concurrent first call stores the same address)
-    }
-    *out = p;
+    static SymbolCache cache;
+    cudaError_t e = symbol_address(cache, g_static_scratch, out);
+    if (e != cudaSuccess) return fail(KF_ECUDA, "cudaGetSymbolAddress(static scratch) failed: %s", cudaGetErrorString(e));
     return KF_OK;
 }
 }  // namespace
