@@ -21,15 +21,16 @@ def climbing(S, D, gain, dtype, hq=4, hkv=2, seed=5):
     return [t.to(dtype).cuda() for t in (q, k, v, gamma, gamma)]
 
 
-@pytest.mark.parametrize("D,variant", [(128, 2), (128, 3), (128, 5), (256, 2), (256, 3)])
+@pytest.mark.parametrize("D,variant,hq", [(128, 2, 4), (128, 3, 4), (128, 3, 2), (128, 5, 4), (256, 2, 4), (256, 3, 4),
+                                          (256, 3, 2)])  # two KV heads: SM pairs at D = 256 with four query heads only
 @pytest.mark.parametrize("S,gain,causal,dtype", [
     (65, 1.0, True, torch.bfloat16),     # one full sub-block and one key
     (700, 1.0, False, torch.float16),    # the base just leaves its threshold
     (700, 3.0, True, torch.bfloat16),    # a move in most sub-blocks, masked ones among them
     (1030, 10.0, False, torch.bfloat16), # scores far above any polynomial's range in a sub-block
 ])
-def test_moving_base_matches_baseline(D, variant, S, gain, causal, dtype):
-    q, k, v, gq, gk = climbing(S, D, gain, dtype)
+def test_moving_base_matches_baseline(D, variant, hq, S, gain, causal, dtype):
+    q, k, v, gq, gk = climbing(S, D, gain, dtype, hq)
     run = lambda val, var: kf.optimized_attention(q, k, val, gq, gk, causal=causal, variant=var).float()
     ref, out = run(v, 1), run(v, variant)
     weight = run(v.abs(), 1)  # sum of p |v|
