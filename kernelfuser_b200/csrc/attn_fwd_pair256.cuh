@@ -6,20 +6,22 @@
 // its own 128-row tile with its own softmax, Q and epilogue warps; the MMAs are tcgen05.mma.cta_group::2 of 256
 // rows, issued by CTA 0 for both, whose B operand (K or V) is split between the two shared memories.
 //
-// What bounds it: at this head dim a CTA of its own streams 64 KB of K and V per 64-key sub-block for 128 query rows, and 148
-// of them pull that from L2 together (~1550 clocks per sub-block where the MMAs take 1024).  A pair copies every K/V
+// What bounds it: at this head dim a CTA of its own streams 64 KB of K and V per 64-key sub-block for 128 query rows, and
+// 148 of them pull that from L2 together (~1550 clocks per sub-block where the MMAs take 1024).  A pair copies every K/V
 // tile once for 256 rows - each CTA loads 32 of the 64 keys of K and half of the columns of V - so the stream halves,
 // and the ring holds five sub-blocks instead of two and a half.  What is left is the chain P V, Q K^T, hand-over,
-// softmax of a score buffer; large launches run at the 1 kW power limit.
-// B200, one CTA per tile -> pairs (back-to-back calls): B=8 S=8192 16/8 heads 3988 -> 3178 us, its 8-GPU shard 509 -> 408.
+// softmax of a score buffer (~1400 clocks per sub-block with everything that a tile adds); large launches run at the
+// 1 kW power limit.  B200, one CTA per tile -> pairs, each by itself back to back: B=8 S=8192 16/8 heads 3917 -> 3556 us;
+// in blocks of 30 ms, its 8-GPU shard 502 -> 459, B=1 S=16384 4/2 heads 473 -> 426.
 //
 // Barriers.  What the issuer waits for lives in CTA 0; what it signals - tcgen05.commit with both CTAs' mask - arrives at
 // the same offset in both.  A K/V stage is full when the halves of both CTAs have landed: each CTA announces its half
 // on CTA 0's barrier and its TMA copy (.cta_group::2, into its own shared memory) completes there, so the barrier that the
 // issuer waits on is that of the copies themselves.  (With a relay in CTA 1 that waits for its copy and tells CTA 0
-// in a release that CTA 0 acquires at cluster scope, B=8 S=8192 16/8 heads took 4750-4900 us against 3178.)  Tensor
-// memory is handed over with relaxed arrivals: tcgen05.wait and tcgen05.fence order its accesses.  Work items are claimed
-// by CTA 0's scheduler and published to both CTAs.
+// in a release that CTA 0 acquires at cluster scope, B=8 S=8192 16/8 heads took 4843 us against 3556; under ncu B=2
+// S=4096 takes 397 k cycles, 407 k with a relay that orders nothing.)  Tensor memory is handed over with relaxed arrivals:
+// tcgen05.wait and tcgen05.fence order its accesses.  Work items are claimed by CTA 0's scheduler and published to both
+// CTAs.
 #pragma once
 #include "attn_fwd_persist256.cuh"
 
@@ -36,7 +38,7 @@ constexpr int kPrItemRing = 8;
 constexpr int kPrSmemBytes = kP2QBytes + kPrRing * kPrStageBytes + 1024 + kPsCtrlBytes;
 static_assert(kPrSmemBytes <= 232448, "shared memory of an SM");
 
-// Pair item `idx` in the order of sg_decode (see ps_decode); `rank` picks the head.
+// Pair item `idx` in the order of sg_decode; `rank` picks the head.
 __device__ __forceinline__ P2Item pr_decode(int idx, uint32_t rank, const AttnArgs& a) {
     P2Item it;
     const int G = a.Hq / a.Hkv, pairs = G / 2;
@@ -218,8 +220,9 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= it.m0);
                 if (!plain || !softmax_ordinary<T, kPolyPairsOneTile, false>(lane_base + col_sb, cs, rs)) {
                     const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                    rs = softmax_general<D, T, kPolyPairsOneTile>(lane_base + col_sb, lane_base + kColO, cs, lim, rs, jj > 0 ? c->pv_done + ((gg - 1) & 1) : nullptr,
-                                               ((gg - 1) >> 1) & 1, s_abort);
+                    rs = softmax_general<D, T, kPolyPairsOneTile>(
+                        lane_base + col_sb, lane_base + kColO, cs, lim, rs,
+                        jj > 0 ? c->pv_done + ((gg - 1) & 1) : nullptr, ((gg - 1) >> 1) & 1, s_abort);
                     if (!rs.ok) { fail = kStatusP2PvDone; break; }
                 }
                 tmem_wait_st();
@@ -375,7 +378,8 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     if (dst == nullptr) return;
 #pragma unroll
                     for (int bx = 0; bx < NB; ++bx)
-                        tma_load_4d_pair(dst + bx * kPrKBoxBytes, &tm_k, full0 + 8 * s, bx * 64, j * kSub + r0 * (kSub / 2), it.kh, it.b);
+                        tma_load_4d_pair(dst + bx * kPrKBoxBytes, &tm_k, full0 + 8 * s, bx * 64, j * kSub + r0 * (kSub / 2),
+                                         it.kh, it.b);
                     if (++s == kPrRing) { s = 0; epar ^= 1; }
                 };
                 auto emit_v = [&](int j, const P2Item& it) {  // all 64 keys, half of the columns
@@ -383,7 +387,8 @@ attn_fwd_pair256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                     if (dst == nullptr) return;
 #pragma unroll
                     for (int bx = 0; bx < NB / 2; ++bx)
-                        tma_load_4d_pair(dst + bx * kPrVBoxBytes, &tm_v, full0 + 8 * s, r0 * (D / 2) + bx * 64, j * kSub, it.kh, it.b);
+                        tma_load_4d_pair(dst + bx * kPrVBoxBytes, &tm_v, full0 + 8 * s, r0 * (D / 2) + bx * 64, j * kSub, it.kh,
+                                         it.b);
                     if (++s == kPrRing) { s = 0; epar ^= 1; }
                 };
                 // (see attn_fwd_persist.cuh: the first K copy waits for the row-prepare this grid may depend on)

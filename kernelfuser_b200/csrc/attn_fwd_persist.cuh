@@ -267,8 +267,9 @@ attn_fwd_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
                 const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= my_m0);
                 if (!plain || !softmax_ordinary<T, kPolyPairsTwoTile, true>(lane_base + col_sb, cs, rs)) {
                     const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                    rs = softmax_general<D, T, kPolyPairsTwoTile>(lane_base + col_sb, lane_base + col_o, cs, lim, rs, jj > 0 ? c->pv_done + 2 * t + ((gg - 1) & 1) : nullptr,
-                                               ((gg - 1) >> 1) & 1, s_abort);
+                    rs = softmax_general<D, T, kPolyPairsTwoTile>(
+                        lane_base + col_sb, lane_base + col_o, cs, lim, rs,
+                        jj > 0 ? c->pv_done + 2 * t + ((gg - 1) & 1) : nullptr, ((gg - 1) >> 1) & 1, s_abort);
                     if (!rs.ok) { fail = kStatusPsPvDone; break; }
                 }
                 // Probe the next score buffer now: the probe is a shared-memory round trip whose latency

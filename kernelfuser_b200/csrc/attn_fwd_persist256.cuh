@@ -1,5 +1,5 @@
-// Persistent, warp-specialised tcgen05 flash-attention forward kernel for head dim 256, one CTA per tile: serves odd numbers
-// of query heads per KV head (even ones run on SM pairs, attn_fwd_pair256.cuh).
+// Persistent, warp-specialised tcgen05 flash-attention forward kernel for head dim 256, one CTA per tile: serves odd
+// numbers of query heads per KV head (even ones run on SM pairs, attn_fwd_pair256.cuh).
 //
 // Same operator and the same inner pipeline as the D = 256 instantiation of attn_fwd_ws256.cuh (reference:
 // `attention_v2_kernel`, src/e1_rope_publication_v1.py:609-649; Q prologue :619-623; rounding contract `_rows`
@@ -51,7 +51,7 @@ struct P2Item {
     int b, h, kh, m0, nsub;
 };
 
-// Tile `idx` in the order of sg_decode (see ps_decode).
+// Tile `idx` in the order of sg_decode (the CTA order of the one-tile kernel).
 __device__ __forceinline__ P2Item p2_decode(int idx, const AttnArgs& a) {
     P2Item it;
     const int G = a.Hq / a.Hkv;
@@ -200,8 +200,9 @@ attn_fwd_persist256_kernel(const __grid_constant__ CUtensorMap tm_q, const __gri
                 const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= it.m0);
                 if (!plain || !softmax_ordinary<T, kPolyPairsOneTile, false>(lane_base + col_sb, cs, rs)) {
                     const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                    rs = softmax_general<D, T, kPolyPairsOneTile>(lane_base + col_sb, lane_base + kColO, cs, lim, rs, jj > 0 ? c->pv_done + ((gg - 1) & 1) : nullptr,
-                                               ((gg - 1) >> 1) & 1, s_abort);
+                    rs = softmax_general<D, T, kPolyPairsOneTile>(
+                        lane_base + col_sb, lane_base + kColO, cs, lim, rs,
+                        jj > 0 ? c->pv_done + ((gg - 1) & 1) : nullptr, ((gg - 1) >> 1) & 1, s_abort);
                     if (!rs.ok) { fail = kStatusP2PvDone; break; }
                 }
                 tmem_wait_st();

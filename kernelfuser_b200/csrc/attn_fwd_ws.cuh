@@ -144,8 +144,9 @@ constexpr uint32_t kPolyPairsOneTile = 0x84210842u, kPolyPairsTwoTile = 0x888448
 
 // ---- softmax of one 64-key sub-block of one row
 // A row's exponent base is the maximum of its first sub-block and from then on of each one with a score more than
-// kGrowLimit above the base, which keeps every probability at or below 2^8.  (Not rounded to a whole number: the
-// row's largest probability is then exactly 1, and in short rows its rounding is most of the error.)
+// kGrowLimit above the base, which keeps every probability at or below 2^8.  (Not rounded to a whole number: as long as
+// no later score exceeds the base, the row's largest probability is then exactly 1, and in short rows its rounding is
+// most of the error.)
 // A row with a NaN score, or a base that is not finite (a score of +inf, or nothing but -inf), comes out NaN: its
 // scores fail the comparison of an ordinary sub-block, and the general one makes the sum NaN.  The probabilities alone
 // would not show it everywhere: the polynomial's clamp turns a NaN into 2^-125.
@@ -199,7 +200,9 @@ template <int D> __device__ __forceinline__ void rescale_output(uint32_t taddr, 
 // P V and multiplies the output so far by alpha.  `ok` is false if that wait failed.
 // Not inlined: these are few of a long row's sub-blocks, and the loop of the others has to stay one short straight run of
 // code.  B200, against the same kernels with mask, maximum and rescale inside the loop (2 s of back-to-back calls):
-// B=16 S=4096 32/8 heads 2358 -> 2320 us, B=1 S=16384 2049 -> 2015 us, B=4 S=2048 193.4 -> 190.8 us.
+// B=16 S=4096 32/8 heads 2358 -> 2320 us, B=1 S=16384 2049 -> 2015 us, B=4 S=2048 193.4 -> 190.8 us.  The call has a
+// price in the persistent kernels, whose loop state is kept across it: D = 128 spills 346 bytes (130 with the function
+// inlined, and yet 2236 -> 2290 us at B=16 S=4096), D = 256 40.
 template <int D, typename T, uint32_t POLY>
 __device__ __noinline__ RowSoftmax softmax_general(uint32_t taddr, uint32_t taddr_o, float c, int lim, RowSoftmax rs,
                                                    uint64_t* prev_pv, uint32_t parity, volatile int* abort_flag) {
@@ -416,8 +419,9 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= tl.m0);
                 if (!plain || !softmax_ordinary<T, kPolyPairsTwoTile, true>(lane_base + col_sb, c, rs)) {
                     const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                    rs = softmax_general<D, T, kPolyPairsTwoTile>(lane_base + col_sb, lane_base + col_o, c, lim, rs, jj > 0 ? pv_done + 2 * t + ((jj - 1) & 1) : nullptr,
-                                               ((jj - 1) >> 1) & 1, s_abort);
+                    rs = softmax_general<D, T, kPolyPairsTwoTile>(
+                        lane_base + col_sb, lane_base + col_o, c, lim, rs,
+                        jj > 0 ? pv_done + 2 * t + ((jj - 1) & 1) : nullptr, ((jj - 1) >> 1) & 1, s_abort);
                     if (!rs.ok) { fail = kStatusWsPvDone; break; }
                 }
                 // Probe the next score buffer now: the probe is a shared-memory round trip whose latency

@@ -218,8 +218,9 @@ attn_fwd_ws1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             const bool plain = jj > 0 && n0 + kSub <= a.S && (!a.causal || n0 + kSub - 1 <= m0);
             if (!plain || !softmax_ordinary<T, kPolyPairsOneTile, D == 128>(lane_base + col_sb, c, rs)) {
                 const int lim = (a.causal ? min(row + 1, a.S) : a.S) - n0;  // keys of this sub-block that the row sees
-                rs = softmax_general<D, T, kPolyPairsOneTile>(lane_base + col_sb, lane_base + kColO, c, lim, rs, jj > 0 ? pv_done + ((jj - 1) & 1) : nullptr,
-                                           ((jj - 1) >> 1) & 1, s_abort);
+                rs = softmax_general<D, T, kPolyPairsOneTile>(
+                    lane_base + col_sb, lane_base + kColO, c, lim, rs, jj > 0 ? pv_done + ((jj - 1) & 1) : nullptr,
+                    ((jj - 1) >> 1) & 1, s_abort);
                 if (!rs.ok) { fail = kStatusWsPvDone; break; }
             }
             tmem_wait_st();

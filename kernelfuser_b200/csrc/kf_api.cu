@@ -481,7 +481,7 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
                      int64_t o_sb, int64_t o_sh, int64_t o_ss, int* status, int variant, int factored, void* stream,
                      const void* gamma_k_full = nullptr, bool after_prepare = false) {
     // after_prepare: the launch before this one in the stream is the row-prepare that wrote `kn`, made by the same
-    // call; small launches of the one-tile kernel then start as its programmatic dependent.
+    // call; the one-tile kernel and the persistent ones then start as its programmatic dependent.
     // gamma_k_full != NULL: `kn` is the RAW key tensor and every K tile is normalised and rotated inside the loop
     // (the reference's mode 'full'); that form exists in the baseline kernel only.
     if (int r = check_common(B, Hq, S, D, dtype)) return r;
@@ -531,14 +531,16 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
     // Automatic choice at D = 128.  The one-tile-per-CTA kernel (two CTAs per SM, groups interleaved heaviest first)
     // fills the SMs, keeps the causal tail short and takes fewest clocks per sub-block; the persistent kernel hides the
     // per-tile fixed costs and its tile pair shares one K/V stream, which also saves power: long launches run at the
-    // 1 kW limit and then at a higher clock (1.51 against 1.45 GHz).  B200, one-tile -> persistent, back to back (in
-    // brackets: alone), by sub-blocks per SM, 32/8 heads unless said:
-    //   3570 B=1 S=16384  1999 -> 1974 us (1738 -> 1712)      2013 B=1 S=12288  1149 -> 1147 ( 984 ->  990)
-    //   3597 B=4 S=8192   2149 -> 2092    (1856 -> 1821)      1827 B=8 S=4096   1208 -> 1185 (1031 -> 1021)
-    //   3542 B=8 S=4096 without mask 2097 -> 2037             1771 B=1 S=8192 without mask 995 -> 1002 (847 -> 864)
-    //   2034 B=4 S=6144   1264 -> 1230    (1077 -> 1066)       913 B=4 S=4096    608 ->  608 ( 518 ->  536)
-    //   2075 B=16 S=3072  1459 -> 1454    (1247 -> 1253)
-    // and 717 -> 824 at B=16 S=2048.  (The factored form exists for kernels 2 and 5 only.)
+    // 1 kW limit and then at a higher clock.  B200, one-tile -> persistent, each kernel by itself for 1.6 s (in short
+    // blocks in turn with another kernel the power that one leaves over shifts either by several per cent), by
+    // sub-blocks per SM, 32/8 heads unless said:
+    //   3570 B=1 S=16384 1967 -> 1942 us     3542 B=4 S=8192 16/4, no mask  1947 -> 1939
+    //   3597 B=4 S=8192  2109 -> 2063        2604 B=1 S=14000 16/8, no mask 1404 -> 1412
+    //   3653 B=16 S=4096 2366 -> 2285        2075 B=16 S=3072               1430 -> 1417
+    //   2013 B=1 S=12288 1138 -> 1129
+    // A call made alone gains less (at 2013 0.6 % slower, at 3570 1.5 % faster).  At B=16 S=2048 717 -> 824.  Items of
+    // two query blocks (odd Hq/Hkv) have only been measured with an earlier softmax loop and stay on the one-tile kernel.
+    // The factored form's line (kernel 2 or 5) is of that time too: at B=16 S=4096 kernel 5 now takes 2193 us, 2 2419.
     if (D == 128 && variant == 0) {
         const long long n_mblk = (S + kf::kBM - 1) / kf::kBM, n_sub_all = (S + kf::kSub - 1) / kf::kSub;
         const long long tiles = (long long)B * Hq * n_mblk;
@@ -554,13 +556,17 @@ int attention_impl(const void* q, const void* kn, const void* v, const void* gam
         // The persistent kernels hide a tile's fixed costs (raw Q copy, transform, copy into TMEM, output store) behind
         // the previous / next tile's main loop, and a pair streams half the K and V; they pay once every SM has enough
         // 64-key sub-blocks to work through and a pair has items to choose from.  B200, one launch item per tile ->
-        // SM pairs, by sub-blocks per SM and items per pair:
-        //   446, 3.5 (B=1 S=16384, 4/2 heads)   473 -> 437 us     62, 6.9 (B=8 S=1024, 16/8)  150 -> 165
-        //   228, 6.9 (B=2 S=4096, 16/8)         315 -> 275        65, 2.6 (B=1 S=3072, 16/8)  101 ->  95
-        //   117, 6.9 (B=4 S=2048, 16/8)         209 -> 192        59, 3.5 (B=4 S=2048, 8/4)   106 -> 105
-        //   114, 3.5 (B=1 S=4096, 16/8)         159 -> 152       112, 1.7 (B=1 S=8192, 4/2)   127 -> 129
-        //    88, 3.0 (B=1 S=3500, 16/8)         129 -> 119        77, 1.4 (B=1 S=6700, 4/2)    98 -> 101
-        // The form of one CTA per tile (odd numbers) pays from about 200 (B=8 S=8192: -11 %; +4 ... +18 % at a hundred).
+        // SM pairs, by sub-blocks per SM and items per pair (us, blocks of 30 ms in turn):
+        //   446, 3.5 (B=1 S=16384, 4/2 heads)   465 -> 426        62, 6.9 (B=8 S=1024, 16/8)  150 -> 162
+        //   228, 6.9 (B=2 S=4096, 16/8)         323 -> 272        64, 2.6 (B=1 S=3072, 16/8)   96 ->  92
+        //   117, 6.9 (B=4 S=2048, 16/8)         205 -> 185        58, 3.5 (B=4 S=2048, 8/4)   103 ->  95
+        //   114, 3.5 (B=1 S=4096, 16/8)         157 -> 145       112, 1.7 (B=1 S=8192, 4/2)   124 -> 125
+        //    87, 3.0 (B=1 S=3500, 16/8)         125 -> 116        77, 1.4 (B=1 S=6700, 4/2)    95 ->  97
+        // without mask: 110, 3.5 (B=2 S=2048, 16/8) 157 -> 139; 110, 6.9 (B=8 S=1024, 16/8) 189 -> 173; 166, 2.6 (B=1
+        // S=4096, 12/6) 198 -> 190.  From 200 also with fewer than two items: 223, 1.7 (B=1 S=16384, 2/1) 231 -> 221;
+        // 249, 1.3 (B=1 S=12288, 2/1, no mask) 307 -> 278.
+        // One CTA per tile (odd numbers), one launch item per tile -> persistent: 176 (B=4 S=2048, 24/8) 291 -> 290; 224
+        // (B=1 S=8192, 8/8) 268 -> 259; 342 (B=2 S=4096, 24/8) 453 -> 402; 456 (B=8 S=4096, 8/8) 644 -> 570.
         const long long n_mblk = (S + kf::kBM - 1) / kf::kBM, n_sub_all = (S + kf::kSub - 1) / kf::kSub;
         const long long per_head = causal ? n_mblk * (n_mblk + 1) : n_mblk * n_sub_all;
         const long long work = (long long)B * Hq * per_head, sms = sm_count();
@@ -722,8 +728,8 @@ int kf_attention_fwd(const void* q, const void* kn, const void* v, const void* g
 }
 
 // The whole operator in one call: row-prepare of K into the caller's `kn`, then the attention kernel - the
-// reference's `launch_attention(mode='query')` (src/e1_rope_publication_v1.py:661-677).  Where the one-tile
-// kernel serves the launch it starts as a programmatic dependent of the prepare (see kDependentMaxTiles).
+// reference's `launch_attention(mode='query')` (src/e1_rope_publication_v1.py:661-677).  The attention kernel starts as
+// a programmatic dependent of the prepare (see kDependentMaxTiles), variants 1 and 2 of D = 128 excepted.
 int kf_optimized_attention(const void* q, const void* k, const void* v, const void* gamma_q, const void* gamma_k,
                            const void* cos_table, const void* sin_table, void* kn, void* out, int B, int Hq, int Hkv,
                            int S, int D, int dtype, int causal, int hf_norm, float eps, float scale, int64_t q_sb,
